@@ -21,7 +21,12 @@
  *    BiCGStab is unpreconditioned); it needs the grid to halve in every
  *    dimension (while all are even) down to at most 4096 cells, and otherwise
  *    runs the PF_MIXED passes.  Both mixed forms converge to the same FP64
- *    tolerance.
+ *    tolerance.  Where every extent is at most 2048 and the tolerance at
+ *    least 1e-12, both first solve the pressure equation directly by FP64
+ *    fast transforms, check the true residual, and iterate (in FP64) only if
+ *    it misses the tolerance; the solve then counts as one iteration.  (Of
+ *    the grids that coarsen, PF_MIXED_MG solves those of more than 2^15 cells
+ *    directly, and none when PF_MG_COOP is set in the environment.)
  */
 #ifndef PYFLOW_B200_H
 #define PYFLOW_B200_H
@@ -55,8 +60,11 @@ enum pf_prec { PF_FP64 = 0, PF_MIXED = 1, PF_MIXED_MG = 2 };
  * forms the solve starts from the DP it is given (for example the previous
  * step's) instead of zero, as the mixed step plans do; the stop criterion is
  * unchanged (max|b - A DP| <= min_res max|b|).  Ignored for PF_FP64, which
- * always starts from DP = 0 like the reference. */
-enum pf_flags { PF_WARM_START = 0x100 };
+ * always starts from DP = 0 like the reference.
+ * PF_DIRECT_SOLVE: PF_FP64 solves directly by fast transforms too (as the
+ * mixed forms do), and runs the reference's BiCGStab only if the result
+ * misses the tolerance. */
+enum pf_flags { PF_WARM_START = 0x100, PF_DIRECT_SOLVE = 0x200 };
 
 /* Result of a Poisson solve (host struct, filled by the synchronous calls). */
 typedef struct pf_solve_info {

@@ -22,8 +22,10 @@ bool grid_ok(const pf_grid* g) {
 
 bool prec_ok(int p) { return p == PF_FP64 || p == PF_MIXED || p == PF_MIXED_MG; }
 
-// prec with the optional PF_WARM_START flag of the solving entry points
-bool prec_flags_ok(int p) { return prec_ok(p & 0xFF) && (p & ~0xFF & ~PF_WARM_START) == 0; }
+// prec with the optional flags of the solving entry points
+bool prec_flags_ok(int p) {
+    return prec_ok(p & 0xFF) && (p & ~0xFF & ~(PF_WARM_START | PF_DIRECT_SOLVE)) == 0;
+}
 
 cudaStream_t S(void* s) { return (cudaStream_t)s; }
 

@@ -1640,6 +1640,8 @@ static cudaError_t mg_attrs() {
     return cudaSuccess;
 }
 
+bool mg_cycles_requested() { return std::getenv("PF_MG_COOP") != nullptr; }
+
 int mg_setup(const pf_grid* g, void* region, MgPlan* P) {
     P->L = mg_levels(g, P->lv, &P->B);
     if (!P->L) return PF_ERR_BAD_ARG;

@@ -43,6 +43,7 @@
 #include "pf_grad.cuh"
 #include "pf_mg.cuh"
 #include "pf_profile.cuh"
+#include "pf_spectral.cuh"
 
 namespace pf {
 
@@ -360,6 +361,79 @@ mixed_residual(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc,
     }
 }
 
+// The direct solve's check: max|b| and max|b - A x| in one sweep, b = (src
+// c1) c2 formed on the fly (16 bytes per cell); nothing is stored.
+struct PhaseCheck {
+    static constexpr int R = 4;
+    const double *x, *src;
+    double c1, c2, mx, mb;
+    struct Raw { double x; };
+    struct Ext { double s; };
+    __device__ Raw raw(long long q, int = 0, int = 0, int = 0) const { return Raw{x[q]}; }
+    __device__ Ext ext(long long q) const { return Ext{src[q]}; }
+    __device__ double op(const Raw& a) const { return a.x; }
+    __device__ void epi(long long, double, double ax, const Raw&, const Ext& e) {
+        const double b = (e.s * c1) * c2;
+        mx = nanmax(mx, fabs(b - ax));
+        mb = nanmax(mb, fabs(b));
+    }
+};
+
+// Ends the direct solve: done when the true residual meets the tolerance,
+// otherwise (a source with a mean, a tolerance below its rounding) FP64
+// BiCGStab passes follow, started from x.  In a graph `cond` is the handle of
+// the IF node that holds them.
+__global__ void __launch_bounds__(kBlock, 2)
+spectral_check(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc, double* part,
+               const double* __restrict__ src, const double* __restrict__ x, double c1, double c2,
+               double min_res, int max_it, int use_cond, cudaGraphConditionalHandle cond) {
+    __shared__ double sh[32];
+    pdl_wait();
+    PhaseCheck ph{x, src, c1, c2, 0.0, 0.0};
+    sweep<double>(d, tl, cf, ph);
+    const double bm = block_max<kBlock>(ph.mx, sh);
+    const double bb = block_max<kBlock>(ph.mb, sh);
+    if (tid0()) { part[blockIdx.x] = bm; part[kMaxPartials + blockIdx.x] = bb; }
+    if (arrive_last(sc)) {
+        const double mx = finish<true>(part, sh);
+        const double mb = finish<true>(part + kMaxPartials, sh);
+        if (tid0()) {
+            const double ratio = mb == 0.0 ? 0.0 : mx / mb;
+            sc->max_b = mb; sc->scale = mx; sc->true_res = mx; sc->max_res = ratio;
+            sc->outer = 1;
+            sc->total = sc->iter = mb == 0.0 ? 0 : 1;
+            sc->use64 = 1; sc->prev_ratio = ratio;
+            bool more = false;
+            if (!(ratio == ratio) || isinf(ratio)) sc->status = PF_NONFINITE;
+            else if (ratio <= min_res) sc->status = PF_OK;
+            else if (max_it <= 1) sc->status = PF_MAXIT;
+            else more = true;
+            sc->done = more ? 0 : 1;
+            sc->counter = 0u;
+            if (use_cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
+        }
+    }
+}
+
+// b = (src c1) c2
+__global__ void __launch_bounds__(kBlock)
+scaled_source(long long n, const double* src, double c1, double c2, double* b) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
+         q += (long long)gridDim.x * blockDim.x)
+        b[q] = (src[q] * c1) * c2;
+}
+
+static void launch_spectral_check(const pf_grid* g, BicgScalars* sc, double* part,
+                                  const double* src, const double* x, double c1, double c2,
+                                  double min_res, int max_it, cudaStream_t s, int use_cond = 0,
+                                  cudaGraphConditionalHandle cond = 0) {
+    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    const Tiling tl = make_tiling(d, 8 * PhaseCheck::R);
+    PF_LAUNCH("spectral_check", s, launch_pdl(spectral_check, dim3(tiled_grid(tl)), dim3(32, 8), 0, s,
+                                              d, tl, lap_coef<double>(g), sc, part, src, x, c1, c2,
+                                              min_res, max_it, use_cond, cond));
+}
+
 // p += DP (src/solver/pressure.py:294)
 __global__ void __launch_bounds__(kBlock)
 add_inplace(long long n, const double* a, double* p) {
@@ -437,12 +511,29 @@ static int run_iterations(const Dims& d, const LapCoef<T>& cf,
     return PF_ERR_CUDA;
 }
 
+// PF_MIXED_MG grids that keep the V-cycle iterations where the direct solve
+// would serve too: all that coarsen when PF_MG_COOP asks for them, and those
+// of at most 2^15 cells.  At 32^3 a captured step takes 0.62 ms with the
+// V-cycles and 0.10 ms with the direct solve, but any change of DP, however
+// small, flips roundings of the FP32 stages, and on these coarse grids (few
+// points per wave, large steps) the two solvers' trajectories part within a
+// request: after 10 steps the velocities differ by 3e-9 (by 8e-15 after the
+// first), against 6e-11 after 5 steps at 128^3 and 7e-11 after 3 at 90x77x63.
+// Requests this small keep the results they have.
+constexpr long long kDirectMinCells = 1LL << 15;
+
+static bool mg_cycles_serve(const pf_grid* g, int prec) {
+    if (prec != PF_MIXED_MG || mg_region_bytes(g) == 0) return false;
+    return mg_cycles_requested() || (long long)g->nx * g->ny * g->nz <= kDirectMinCells;
+}
+
 int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
                    double min_res, int max_it, const double* source,
                    double* DP, double* p, void* ws, cudaStream_t s,
                    pf_solve_info* info) {
     // PF_WARM_START (mixed forms): the refinement starts from the DP given
-    const bool warm = (prec & PF_WARM_START) != 0 && (prec & 0xFF) != PF_FP64;
+    bool warm = (prec & PF_WARM_START) != 0 && (prec & 0xFF) != PF_FP64;
+    const bool direct = (prec & PF_DIRECT_SOLVE) != 0 || (prec & 0xFF) != PF_FP64;
     prec &= 0xFF;
     Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
     const size_t n = (size_t)d.n;
@@ -458,7 +549,31 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
     pf_solve_info out{0.0, 0, 1, PF_OK};
     // the reference loop always runs at least one iteration
     max_it = std::max(max_it, 1);
-    if (prec == PF_FP64) {
+    bool solved = false, use64 = false;
+    int outer = 0, total = 0;
+    if (direct && !mg_cycles_serve(g, prec) && spectral_applies(g, min_res, DP, ptr)) {
+        // the tables sit in the region of the iterative solver's vectors
+        SpectralPlan sp;
+        if (spectral_setup(g, ptr, &sp) != cudaSuccess ||
+            spectral_enqueue_tables(sp, s) != cudaSuccess ||
+            spectral_enqueue_solve(sp, source, c1 * c2, DP, s) != cudaSuccess)
+            return PF_ERR_CUDA;
+        launch_spectral_check(g, sc, part, source, DP, c1, c2, min_res, max_it, s);
+        if (cudaGetLastError() != cudaSuccess || read_scalars(sc, &hs, s)) return PF_ERR_CUDA;
+        solved = hs.done != 0;
+        outer = hs.max_b == 0.0 ? 0 : 1;
+        total = hs.total;
+        out.max_res = hs.max_res; out.iterations = total; out.outer = outer; out.status = hs.status;
+        // a non-finite right-hand side leaves DP = 0, as the iterations do
+        if (hs.status == PF_NONFINITE &&
+            cudaMemsetAsync(DP, 0, n * sizeof(double), s) != cudaSuccess)
+            return PF_ERR_CUDA;
+        // the mixed forms go on from here, in FP64; PF_FP64 starts over
+        warm = use64 = prec != PF_FP64;
+    }
+    if (solved) {
+        // nothing more to iterate
+    } else if (prec == PF_FP64) {
         BicgVecs<double> v = carve<double>(ptr, n);
         const LapCoef<double> cf = lap_coef<double>(g);
         PF_LAUNCH("bicg_init_f64", s, bicg_init<double, false><<<gp, kBlock, 0, s>>>(
@@ -500,8 +615,7 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
                                                                        warm ? nullptr : DP, nullptr));
         if (read_scalars(sc, &hs, s)) return PF_ERR_CUDA;
         const double max_b = hs.max_b;
-        int status = PF_OK, outer = 0, total = 0;
-        bool use64 = false;
+        int status = PF_OK;
         double ratio = max_b > 0 ? 1.0 : 0.0, prev_ratio = 2.0;
         if (!(max_b == max_b)) status = PF_NONFINITE;
         while (status == PF_OK && max_b > 0.0) {
@@ -985,8 +1099,10 @@ size_t step_plan_ws_bytes(const pf_grid* g, int prec) {
     // PF_MIXED_MG: the coarsest level's pseudo-inverse in a slot of its own
     // (the region r is reused by the predictor every step), computed once
     const size_t pinv = prec == PF_MIXED_MG ? kPlanPinvBytes + kMgBarrierBytes : 0;
+    // mixed forms: the direct solve's tables, filled once too
+    const size_t tables = prec == PF_FP64 ? 0 : spectral_table_bytes(g);
     return align256(n * sizeof(double)) + align256(sizeof(BicgScalars)) +
-           align256(kNumPartials * kMaxPartials * sizeof(double)) + align256(r) + pinv;
+           align256(kNumPartials * kMaxPartials * sizeof(double)) + align256(r) + tables + pinv;
 }
 
 // Pointers of one request's plan workspace (see step_plan_ws_bytes).
@@ -1001,9 +1117,11 @@ struct PlanLayout {
     float* e32;
     double *bb, *rr;
     MgPlan mg;
+    SpectralPlan sp;  // on: the direct solve, with FP64 passes behind it
 };
 
-static int plan_layout(const pf_grid* g, int prec, void* ws, PlanLayout* L) {
+static int plan_layout(const pf_grid* g, int prec, double min_res, const double* DP, void* ws,
+                       PlanLayout* L) {
     L->d = Dims{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
     const size_t n = (size_t)L->d.n;
     char* ptr = (char*)ws;
@@ -1019,9 +1137,16 @@ static int plan_layout(const pf_grid* g, int prec, void* ws, PlanLayout* L) {
     L->e32 = (float*)vp;
     L->bb = (double*)(L->R + 9 * align256(n * sizeof(double)));
     L->rr = (double*)(L->R + 10 * align256(n * sizeof(double)));
+    L->mg = MgPlan();
+    L->sp = SpectralPlan();
+    if (prec != PF_FP64 && !mg_cycles_serve(g, prec)) {
+        char* tables = (char*)ws + step_plan_ws_bytes(g, prec) - spectral_table_bytes(g) -
+                       (prec == PF_MIXED_MG ? kPlanPinvBytes + kMgBarrierBytes : 0);
+        if (spectral_applies(g, min_res, DP, tables))
+            return spectral_setup(g, tables, &L->sp) == cudaSuccess ? PF_OK : PF_ERR_CUDA;
+    }
     // PF_MIXED_MG: multigrid-preconditioned inner passes when the grid
     // coarsens (vectors in the region of the FP32 solver vectors)
-    L->mg = MgPlan();
     if (prec == PF_MIXED_MG && mg_region_bytes(g) <= 9 * align256(n * sizeof(double))) {
         const int e = mg_setup(g, L->R, &L->mg);
         if (e != PF_OK && e != PF_ERR_BAD_ARG) return e;
@@ -1055,8 +1180,33 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
     int rc = PF_OK;
     // ---- divergence, solver set-up
     cudaGraph_t seg1 = nullptr;
+    cudaGraph_t C = G;        // the graph that holds the solver's loops
+    cudaGraphNode_t nsolved;  // the node after which DP is final
+    cudaGraphConditionalHandle hmore = 0;
+    if (P.sp.on && cudaGraphConditionalHandleCreate(&hmore, G, 0, cudaGraphCondAssignDefault) !=
+                       cudaSuccess)
+        return PF_ERR_CUDA;
     if ((rc = capture_begin(cs, nullptr))) return rc;
     launch_div(g, u, v, w, P.div, cs);
+    if (P.sp.on) {
+        // the direct solve and its check; the refinement loop below, with FP64
+        // passes only, sits in an IF node that the check opens
+        spectral_enqueue_solve(P.sp, P.div, c1 * c2, DP, cs);
+        launch_spectral_check(g, sc, part, P.div, DP, c1, c2, min_res, max_it, cs, 1, hmore);
+        if ((rc = capture_end(cs, &seg1))) return rc;
+        cudaGraphNode_t ns;
+        rc = add_child(G, dep, seg1, &ns);
+        cudaGraphDestroy(seg1);
+        if (rc) return rc;
+        cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
+        prm.conditional.handle = hmore;
+        prm.conditional.type = cudaGraphCondTypeIf;
+        prm.conditional.size = 1;
+        if (cudaGraphAddNode(&nsolved, G, &ns, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
+        C = prm.conditional.phGraph_out[0];
+        dep = nullptr;
+        if ((rc = capture_begin(cs, nullptr))) return rc;
+    }
     if (prec == PF_FP64) {
         const LapCoef<double> cf = lap_coef<double>(g);
         const Tiling ta = make_tiling(d, 8 * PhaseCA<double>::R);
@@ -1068,18 +1218,22 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
         // first step): its first residual is r = b - A DP, and the stop test
         // stays the reference's, max|b - A DP| <= min_res max|b|
         const Tiling tld = make_tiling(d, 8 * PhaseResidual::R);
-        mixed_b_init<<<gp, kBlock, 0, cs>>>(d, sc, part, P.div, c1, c2, P.bb, nullptr, nullptr);
+        if (P.sp.on)
+            scaled_source<<<gp, kBlock, 0, cs>>>(d.n, P.div, c1, c2, P.bb);
+        else
+            mixed_b_init<<<gp, kBlock, 0, cs>>>(d, sc, part, P.div, c1, c2, P.bb, nullptr, nullptr);
         mixed_residual<<<tiled_grid(tld), blk2, 0, cs>>>(d, tld, lap_coef<double>(g), sc, part,
                                                         P.bb, DP, P.rr);
     }
     if ((rc = capture_end(cs, &seg1))) return rc;
     cudaGraphNode_t n1, nw;
-    rc = add_child(G, dep, seg1, &n1);
+    rc = add_child(C, dep, seg1, &n1);
     cudaGraphDestroy(seg1);
     if (rc) return rc;
     cudaGraph_t body;
     cudaGraphConditionalHandle h;
-    if ((rc = add_while(G, n1, &nw, &body, &h))) return rc;
+    if ((rc = add_while(C, n1, &nw, &body, &h))) return rc;
+    if (!P.sp.on) nsolved = nw;
     if (prec == PF_FP64) {
         const LapCoef<double> cf = lap_coef<double>(g);
         const Tiling ta = make_tiling(d, 8 * PhaseCA<double>::R);
@@ -1104,12 +1258,6 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
         const LapCoef<double> cf64 = lap_coef<double>(g);
         const Tiling ta64 = make_tiling(d, 8 * PhaseCA<double>::R);
         const Tiling tb64 = make_tiling(d, 8 * PhaseB<double>::R);
-        // outer body: branch kernel, IF(use64) {FP64 pass} ELSE {FP32 pass},
-        // then fold + residual + control
-        cudaGraphConditionalHandle h32, h64, hif;
-        if (cudaGraphConditionalHandleCreate(&hif, body, 0, cudaGraphCondAssignDefault) !=
-                cudaSuccess)
-            return PF_ERR_CUDA;
         // a one-thread kernel node: func(args...) with the given argument list
         auto add_tiny = [](cudaGraph_t gr, void* func, void** args, cudaGraphNode_t* node) {
             cudaKernelNodeParams kp;
@@ -1121,34 +1269,26 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
             return cudaGraphAddKernelNode(node, gr, nullptr, 0, &kp) == cudaSuccess ? PF_OK
                                                                                      : PF_ERR_CUDA;
         };
-        cudaGraphNode_t b0, bif, b3;
-        {
-            BicgScalars* scp = sc;
-            void* args[] = {&scp, &hif};
-            if ((rc = add_tiny(body, (void*)pass_branch, args, &b0))) return rc;
-        }
-        cudaGraph_t br64, br32;
-        {
-            cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
-            prm.conditional.handle = hif;
-            prm.conditional.type = cudaGraphCondTypeIf;
-            prm.conditional.size = 2;
-            if (cudaGraphAddNode(&bif, body, &b0, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
-            br64 = prm.conditional.phGraph_out[0];
-            br32 = prm.conditional.phGraph_out[1];
-        }
-        // FP32 branch: re-arm its loop, set-up, then the inner WHILE (the
-        // handle belongs to the branch graph that holds the loop)
-        {
+        // One pass in graph `gr`: re-arm its loop, set-up, then the inner
+        // WHILE (its handle belongs to the graph that holds the loop).  The
+        // FP64 pass runs to the remaining tolerance.
+        auto add_pass = [&](cudaGraph_t gr, bool f64, cudaGraphNode_t* cw) -> int {
             cudaGraph_t pre = nullptr, inner_body = nullptr;
-            cudaGraphNode_t a0, c1n, cw;
-            if (cudaGraphConditionalHandleCreate(&h32, br32, 1, cudaGraphCondAssignDefault) !=
+            cudaGraphNode_t a0, c1n;
+            cudaGraphConditionalHandle hp;
+            if (cudaGraphConditionalHandleCreate(&hp, gr, 1, cudaGraphCondAssignDefault) !=
                 cudaSuccess)
                 return PF_ERR_CUDA;
-            void* args[] = {&h32};
-            if ((rc = add_tiny(br32, (void*)arm_condition, args, &a0))) return rc;
-            if ((rc = capture_begin(cs, nullptr))) return rc;
-            if (mg.L) {
+            void* args[] = {&hp};
+            int rc = add_tiny(gr, (void*)arm_condition, args, &a0);
+            if (rc || (rc = capture_begin(cs, nullptr))) return rc;
+            if (f64) {
+                bicg_init<double, true><<<gp, kBlock, 0, cs>>>(d, sc, part, P.rr, 0.0, 0.0, v64,
+                                                              e64, max_it, 0.5);
+                pass_tol64<<<1, 32, 0, cs>>>(sc, min_res);
+                bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64,
+                                                                  e64);
+            } else if (mg.L) {
                 mg_enqueue_init(mg, sc, part, P.rr, kInnerTol, max_it, cs, min_res);
             } else {
                 bicg_init<float, true><<<gp, kBlock, 0, cs>>>(d, sc, part, P.rr, 0.0, 0.0, P.v32,
@@ -1157,47 +1297,49 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
                                                                P.e32);
             }
             if ((rc = capture_end(cs, &pre))) return rc;
-            rc = add_child(br32, a0, pre, &c1n);
+            rc = add_child(gr, a0, pre, &c1n);
             cudaGraphDestroy(pre);
             if (rc) return rc;
-            if ((rc = add_while(br32, c1n, &cw, &inner_body, &h32, false))) return rc;
+            if ((rc = add_while(gr, c1n, cw, &inner_body, &hp, false))) return rc;
             if ((rc = capture_begin(cs, inner_body))) return rc;
-            if (mg.L) {
+            if (f64) {
+                bicg_b<double><<<tiled_grid(tb64), blk2, 0, cs>>>(d, tb64, cf64, sc, part, v64, 1,
+                                                                 hp);
+                bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64,
+                                                                  e64, 1, hp);
+            } else if (mg.L) {
                 // two iterations per pass of the body: the p buffers alternate
-                mg_enqueue_iteration(mg, sc, part, 0, cs, 1, h32);
-                mg_enqueue_iteration(mg, sc, part, 1, cs, 1, h32);
+                mg_enqueue_iteration(mg, sc, part, 0, cs, 1, hp);
+                mg_enqueue_iteration(mg, sc, part, 1, cs, 1, hp);
             } else {
-                bicg_b<float><<<tiled_grid(tb), blk2, 0, cs>>>(d, tb, cf, sc, part, P.v32, 1,
-                                                              h32);
+                bicg_b<float><<<tiled_grid(tb), blk2, 0, cs>>>(d, tb, cf, sc, part, P.v32, 1, hp);
                 bicg_ca<float><<<tiled_grid(ta), blk2, 0, cs>>>(d, ta, cf, sc, part, P.v32,
-                                                               P.e32, 1, h32);
+                                                               P.e32, 1, hp);
             }
-            if ((rc = capture_end(cs, &inner_body))) return rc;
-        }
-        // FP64 branch: re-arm, set-up with the remaining tolerance, its WHILE
-        {
-            cudaGraph_t pre = nullptr, inner_body = nullptr;
-            cudaGraphNode_t a0, c1n, cw;
-            if (cudaGraphConditionalHandleCreate(&h64, br64, 1, cudaGraphCondAssignDefault) !=
-                cudaSuccess)
+            return capture_end(cs, &inner_body);
+        };
+        cudaGraphNode_t bif, b3;
+        if (P.sp.on) {
+            // behind the direct solve only FP64 passes make sense
+            if ((rc = add_pass(body, true, &bif))) return rc;
+        } else {
+            // outer body: branch kernel, IF(use64) {FP64 pass} ELSE {FP32 pass},
+            // then fold + residual + control
+            cudaGraphConditionalHandle hif;
+            if (cudaGraphConditionalHandleCreate(&hif, body, 0, cudaGraphCondAssignDefault) !=
+                    cudaSuccess)
                 return PF_ERR_CUDA;
-            void* args[] = {&h64};
-            if ((rc = add_tiny(br64, (void*)arm_condition, args, &a0))) return rc;
-            if ((rc = capture_begin(cs, nullptr))) return rc;
-            bicg_init<double, true><<<gp, kBlock, 0, cs>>>(d, sc, part, P.rr, 0.0, 0.0, v64, e64,
-                                                          max_it, 0.5);
-            pass_tol64<<<1, 32, 0, cs>>>(sc, min_res);
-            bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64, e64);
-            if ((rc = capture_end(cs, &pre))) return rc;
-            rc = add_child(br64, a0, pre, &c1n);
-            cudaGraphDestroy(pre);
-            if (rc) return rc;
-            if ((rc = add_while(br64, c1n, &cw, &inner_body, &h64, false))) return rc;
-            if ((rc = capture_begin(cs, inner_body))) return rc;
-            bicg_b<double><<<tiled_grid(tb64), blk2, 0, cs>>>(d, tb64, cf64, sc, part, v64, 1, h64);
-            bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64, e64,
-                                                              1, h64);
-            if ((rc = capture_end(cs, &inner_body))) return rc;
+            cudaGraphNode_t b0, cw;
+            BicgScalars* scp = sc;
+            void* args[] = {&scp, &hif};
+            if ((rc = add_tiny(body, (void*)pass_branch, args, &b0))) return rc;
+            cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
+            prm.conditional.handle = hif;
+            prm.conditional.type = cudaGraphCondTypeIf;
+            prm.conditional.size = 2;
+            if (cudaGraphAddNode(&bif, body, &b0, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
+            if ((rc = add_pass(prm.conditional.phGraph_out[1], false, &cw))) return rc;
+            if ((rc = add_pass(prm.conditional.phGraph_out[0], true, &cw))) return rc;
         }
         cudaGraph_t post = nullptr;
         if ((rc = capture_begin(cs, nullptr))) return rc;
@@ -1217,7 +1359,7 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
     launch_vel_corr(g, DP, dt / rho, u, v, w, cs);
     launch_stats(g, u, v, w, stats, P.R, cs);
     if ((rc = capture_end(cs, &seg3))) return rc;
-    rc = add_child(G, nw, seg3, end);
+    rc = add_child(G, nsolved, seg3, end);
     cudaGraphDestroy(seg3);
     return rc;
 }
@@ -1287,17 +1429,17 @@ int step_plan_create(const pf_grid* g, int prec, int rk4, double* u, double* v,
                      double dt, double min_res, int max_it, const pf_step_closure* c,
                      void* ws, double* stats, void** out) {
     PlanLayout P;
-    int rc = plan_layout(g, prec, ws, &P);
+    int rc = plan_layout(g, prec, min_res, DP, ws, &P);
     if (rc != PF_OK) return rc;
     if (predictor_prepare(prec) != cudaSuccess) return PF_ERR_CUDA;
     if (c && c->kind == PF_CLOSURE_MLP && mlp_prepare() != cudaSuccess) return PF_ERR_CUDA;
     cudaStream_t cs;
     if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) return PF_ERR_CUDA;
-    if (P.mg.L) {
-        if (mg_enqueue_setup(P.mg, cs) != PF_OK || cudaStreamSynchronize(cs) != cudaSuccess) {
-            cudaStreamDestroy(cs);
-            return PF_ERR_CUDA;
-        }
+    if ((P.mg.L && mg_enqueue_setup(P.mg, cs) != PF_OK) ||
+        (P.sp.on && spectral_enqueue_tables(P.sp, cs) != cudaSuccess) ||
+        cudaStreamSynchronize(cs) != cudaSuccess) {
+        cudaStreamDestroy(cs);
+        return PF_ERR_CUDA;
     }
     prof_suspend(true);
     StepPlan* plan = new StepPlan();
@@ -1343,7 +1485,8 @@ int batch_plan_create(int prec, int rk4, const pf_batch_member* m, int count, vo
     if (count < 1 || count > kMaxBatch) return PF_ERR_BAD_ARG;
     PlanLayout* P = new PlanLayout[count];
     int rc = PF_OK;
-    for (int r = 0; r < count && rc == PF_OK; ++r) rc = plan_layout(&m[r].grid, prec, m[r].ws, &P[r]);
+    for (int r = 0; r < count && rc == PF_OK; ++r) 
+        rc = plan_layout(&m[r].grid, prec, m[r].min_res, m[r].DP, m[r].ws, &P[r]);
     if (rc != PF_OK) { delete[] P; return rc; }
     // the requests' solves run as parallel branches: their mid levels stay on
     // the per-level kernels (no grid-barrier launches that could wait on one
@@ -1365,7 +1508,9 @@ int batch_plan_create(int prec, int rk4, const pf_batch_member* m, int count, vo
     // member carried over from an earlier plan may still be computing there
     // and is not touched
     for (int r = 0; r < count && rc == PF_OK; ++r)
-        if (m[r].fresh && P[r].mg.L && mg_enqueue_setup(P[r].mg, cs) != PF_OK) rc = PF_ERR_CUDA;
+        if (m[r].fresh && ((P[r].mg.L && mg_enqueue_setup(P[r].mg, cs) != PF_OK) ||
+                           (P[r].sp.on && spectral_enqueue_tables(P[r].sp, cs) != cudaSuccess)))
+            rc = PF_ERR_CUDA;
     if (rc == PF_OK && cudaStreamSynchronize(cs) != cudaSuccess) rc = PF_ERR_CUDA;
     StepPlan* plan = new StepPlan();
     prof_suspend(true);

@@ -1,0 +1,102 @@
+"""The direct pressure solve by fast transforms (mixed forms; PF_FP64 with
+PF_DIRECT_SOLVE): against numpy's FFT of the same operator in FP64 over
+extents of every radix, primes, odd pairs and both ends of the range; its
+check; and the iterations behind it."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# powers of two (every last radix), 3, 5, 7 and other primes, odd extents in
+# each position (unpaired and unaligned lines), two-cell axes, long lines
+SHAPES = [(2, 2, 2), (3, 2, 5), (8, 4, 2), (16, 32, 64), (64, 16, 32), (12, 20, 28), (9, 25, 49),
+          (15, 7, 33), (21, 34, 11), (13, 17, 19), (31, 6, 10), (10, 37, 5), (6, 10, 61),
+          (128, 4, 6), (4, 256, 6), (4, 6, 512), (1024, 3, 4), (2, 1024, 6), (4, 2, 2048),
+          (2048, 2, 3), (3, 2048, 2), (96, 80, 72), (4, 1331, 3), (2, 3, 1021), (2039, 2, 2)]
+
+
+def _solve(src, sp, prec, tol=1e-10, max_it=20000, rho=1.3, dt=0.01, flags=0):
+    import pyflow_b200._lib as L
+    import pyflow_b200.ops as ops
+    DP = torch.full_like(src, 7.0)
+    p = torch.ones_like(src)
+    g = ops.grid(src.shape, sp)
+    pr = ops.PREC[prec]
+    ws = ops.workspace(g, pr, src.device)
+    info = L.SolveInfo()
+    L.check("pf_bicgstab_solve", L.lib().pf_bicgstab_solve(
+        ctypes.byref(g), pr | flags, rho, dt, tol, max_it, ops._p(src), ops._p(DP), ops._p(p),
+        ops._p(ws), ws.numel(), ops._stream(src), ctypes.byref(info)))
+    return DP, p, info
+
+
+def _exact(src, sp, rho=1.3, dt=0.01):
+    """Zero-mean solution of the 7-point Laplacian by numpy's FFT."""
+    lam = 0.0
+    for d, n in enumerate(src.shape):
+        s = [1, 1, 1]
+        s[d] = n
+        lam = lam - (4.0 / sp[d] ** 2 * np.sin(np.pi * np.arange(n) / n) ** 2).reshape(s)
+    lam[0, 0, 0] = 1.0
+    h = np.fft.fftn(src) / lam
+    h[0, 0, 0] = 0.0
+    return np.fft.ifftn(h).real * (rho / dt)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_direct_solve_matches_fft(shape):
+    """FP64 transforms leave a few roundings (2e-16) per stage relative to the
+    norm, direct sums of a prime p up to p: 1e-12 of the norm bounds both."""
+    rng = np.random.default_rng(sum(shape))
+    sp = (0.31, 0.17, 0.23)
+    src = rng.standard_normal(shape)
+    src -= src.mean()
+    want = _exact(src, sp)
+    forms = [("mixed", 0), ("fp64", 0x200)]
+    if np.prod(shape) > 2 ** 15:
+        forms.append(("mixed_mg", 0))   # smaller grids that coarsen keep the V-cycles
+    for prec, flags in forms:
+        DP, p, info = _solve(torch.tensor(src, device="cuda"), sp, prec, flags=flags)
+        assert info.status == 0 and info.iterations == 1 and info.max_res <= 1e-10
+        got = DP.cpu().numpy()
+        assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+        assert torch.equal(p, 1.0 + DP)
+
+
+def test_source_with_a_mean_goes_on_iterating():
+    """A right-hand side with a mean has no solution: the direct result
+    misses the tolerance, the FP64 passes run to the limit and say so."""
+    src = torch.ones(16, 12, 20, dtype=torch.float64, device="cuda")
+    src[3, 4, 5] = 2.0
+    for prec, flags in (("mixed", 0), ("mixed_mg", 0), ("fp64", 0x200)):
+        _, _, info = _solve(src, (0.1,) * 3, prec, max_it=40, flags=flags)
+        assert info.status != 0 and info.max_res > 1e-10 and info.iterations >= 1
+
+
+def test_tight_tolerance_iterates():
+    """Below the direct solve's own rounding the iterations run as before."""
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal((24, 24, 24))
+    src = torch.tensor(a - a.mean(), device="cuda")
+    _, _, info = _solve(src, (0.1,) * 3, "mixed", tol=2e-13)
+    assert info.iterations > 1
+
+
+def test_unaligned_fields():
+    """Fields that start 8 bytes off a 16-byte boundary, even extents."""
+    import pyflow_b200.ops as ops
+    shape, sp = (16, 12, 10), (0.31, 0.17, 0.23)
+    n = int(np.prod(shape))
+    rng = np.random.default_rng(9)
+    a = rng.standard_normal(shape)
+    a -= a.mean()
+    buf = [torch.zeros(n + 1, dtype=torch.float64, device="cuda") for _ in range(3)]
+    src, DP, p = (b[1:].view(shape) for b in buf)
+    src.copy_(torch.tensor(a, device="cuda"))
+    info = ops.bicgstab_solve(src, DP, p, sp, 1.3, 0.01, 1e-10, 100, prec="mixed")
+    want = _exact(a, sp)
+    assert info.status == 0
+    assert np.linalg.norm(DP.cpu().numpy() - want) <= 1e-12 * np.linalg.norm(want)
