@@ -61,24 +61,24 @@ def sfs_adjoint_accumulate(lam, spacing, weight, out):
 
 
 def project(vel, spacing, rho, dt, tol=1e-12, max_it=20000, p=None, DP=None):
-    """In-place projection P vel = vel - G L^-1 D vel (FP64 BiCGStab): the
-    target-data corrector Domain.TargetDataVelCorr (src/data/domain.py:445-468),
+    """In-place projection P vel = vel - G L^-1 D vel (FP64, solved directly):
+    the target-data corrector Domain.TargetDataVelCorr (src/data/domain.py:445-468),
     divergence, pressure solve from DP = 0, vel -= dt/rho grad DP.  The
     reference's solve also adds DP to the pressure it is given (the
     simulation's p): pass ``p`` to get that; ``DP`` receives the solution."""
     u, v, w = vel
-    src = ops.div_vel(u, v, w, spacing)
     DP = torch.zeros_like(u) if DP is None else DP.zero_()
     p = torch.zeros_like(u) if p is None else p
     # a field that is already divergence free to the solver's precision (the
     # adjoint of a loss between two projected fields: its divergence is
-    # round-off of the field) needs no correction: BiCGStab on a round-off
-    # right-hand side only iterates on noise, stagnates at the relative
-    # tolerance and can end non-finite
-    vmax = max(float(t.abs().max()) for t in vel)
-    if float(src.abs().max()) <= 1e-9 * vmax / min(spacing):
+    # round-off of the field) needs no correction: a solve of a round-off
+    # right-hand side (whose mean is not zero) only iterates on noise,
+    # stagnates at the relative tolerance and can end non-finite
+    mu, mv, mw, _, mdiv = ops.stats(u, v, w, spacing).tolist()
+    if mdiv <= 1e-9 * max(mu, mv, mw) / min(spacing):
         return None
-    info = ops.bicgstab_solve(src, DP, p, spacing, rho, dt, tol, max_it)
+    src = ops.div_vel(u, v, w, spacing)
+    info = ops.bicgstab_solve(src, DP, p, spacing, rho, dt, tol, max_it, direct=True)
     if info.status == L.PF_NONFINITE:
         raise RuntimeError("projection solve: non-finite residual")
     ops.vel_corr(DP, dt / rho, u, v, w, spacing)
@@ -191,7 +191,7 @@ def step_vjp(state, lam_out, spacing, mu, rho, dt, sfs=None, rk4=True,
 class ForwardStep(torch.autograd.Function):
     """One Domain.forwardStep on (u, v, w) as a differentiable map.
 
-    forward: pf_forward_step (FP64, BiCGStab to ``tol``); backward: the
+    forward: pf_forward_step (FP64, solved directly to ``tol``); backward: the
     hand-written adjoint above, recomputing the RK4 stages from the saved
     input.  ``sfs`` (6, nx, ny, nz) stresses, if given, are an input too."""
 
@@ -214,7 +214,7 @@ class ForwardStep(torch.autograd.Function):
         p = torch.zeros_like(uo)
         DP = torch.zeros_like(uo)
         info = ops.forward_step(uo, vo, wo, p, DP, spacing, mu, rho, dt, rk4=rk4,
-                                min_res=tol, max_it=max_it, sfs=sd)
+                                min_res=tol, max_it=max_it, sfs=sd, direct=True)
         if info.status == L.PF_NONFINITE:
             raise RuntimeError("forward step: non-finite pressure residual")
         return uo, vo, wo
