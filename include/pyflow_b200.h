@@ -366,6 +366,16 @@ int pf_slab_bicg_init(const pf_grid* g, int halo, double rho, double dt,
 int pf_slab_bicg_phase(const pf_grid* g, int halo, int phase, const double* recv,
                        int world, double* DP, void* ws, double* send, void* stream);
 int pf_slab_bicg_info(const pf_grid* g, void* ws, double* info, void* stream);
+/* The whole solve for `count` slabs held by one process on one device, in
+ * rank order (g[r], div[r], DP[r], ws[r], ws_bytes[r], send[r] as for
+ * pf_slab_bicg_init): bitwise what the loop above gives, without
+ * exchanges or gathers, as one cooperative launch per 256 iterations.
+ * Synchronous.  PF_ERR_TOO_LARGE, with nothing changed: more than 24 slabs,
+ * no cooperative launch, or per-kernel timing on (run the phases). */
+int pf_slab_local_solve(int count, const pf_grid* g, int halo, double rho, double dt,
+                        double min_res, int max_it, const double* const* div,
+                        double* const* DP, void* const* ws, const size_t* ws_bytes,
+                        double* const* send, void* stream, pf_solve_info* info);
 int pf_slab_add(const pf_grid* g, int halo, const double* DP, double* p, void* stream);
 
 /* NGA restart I/O from device memory (readNGArestart / writeNGArestart,

@@ -31,9 +31,11 @@
 //           APPLY_S -> gather -> FINAL -> gather -> P (folds the stop test)
 // until the stop flag is set; then p += DP (pf_slab_add) and, after an
 // exchange of DP, the projection.
+#include <algorithm>
 #include <cmath>
 
 #include "pf_common.cuh"
+#include "pf_gridbar.cuh"
 #include "pf_kernels.cuh"
 #include "pf_profile.cuh"
 #include "pf_sweep.cuh"
@@ -340,6 +342,353 @@ int apply_blocks(const Slab& sl) {
     return (int)std::max<long long>(1, std::min<long long>(nt, std::min(num_sms() * 8, kMaxPartials)));
 }
 
+
+// --------------------------------------------------- all slabs in one process
+// The whole solve of R slabs held by one process as one cooperative launch
+// (per kGroupIters iterations).  Driven from the host, an iteration is 16
+// launches and copies per slab.  Per iteration, phases -> this kernel, on one
+// B200: two slabs of 48x64x64 270 -> 28.7 us, three of 16x40x40 383 -> 19.4,
+// two of 64x128x128 277 -> 97, two of 128x256x256 835 -> 759.  What is left at
+// the small sizes is latency: each grid barrier with its fold takes 3.5 us,
+// and after it every load goes to L2.  An iteration is three phases separated
+// by grid barriers:
+//   P1  pp' = (pp - omega vv) beta + res at the seven points, vv' = A pp',
+//       (vv', res0)
+//   P2  s = res - alpha vv' at the seven points, t = A s, (s,t), (t,t)
+//       (and DP += alpha pp' while the barrier behind it is under way)
+//   P3  DP += omega s, res = s - omega t, (res,res0), max|res|
+// The x neighbours of a slab's end planes are read where they lie, in the
+// next slab, so nothing is exchanged; pp and vv alternate between two buffers
+// each (the phase kernels' s and the just-consumed t are the second ones).
+// Every element's operations, and every sum -- per virtual block of the phase
+// kernels' grids, then blocks in block order, then slabs in rank order, which
+// each physical block folds for itself -- are those of the phase kernels, so
+// the solve is bitwise the one the phases give.
+constexpr int kGroupMax = 24;     // slabs of one launch (its arguments are passed by value)
+constexpr int kGroupIters = 256;  // iterations per launch
+constexpr int kGroupParts = kSlabVals * kMaxPartials / 5;  // partial slots per sum and slab
+
+struct GroupSlab {
+    int nxl, ab, nb;  // interior planes; virtual blocks of the operator and the pointwise phases
+    double *res, *res0, *pp[2], *vv[2], *DP, *part;
+    const double* send;
+    SlabScalars* sc;
+};
+
+struct Group {
+    int R, h, ny, nz;
+    int nab, nnb;  // virtual blocks over all slabs
+    int one;       // every virtual block of the operator is one tile
+    LapCoef<double> cf;
+    unsigned* bar;
+    GroupSlab s[kGroupMax];
+};
+
+// A physical block is four groups of 256 threads, each working through
+// virtual blocks on its own (named barriers 1-4); the grid barrier then has
+// 148 arrivals instead of 592.
+constexpr int kGroups = 4;
+
+__device__ __forceinline__ void group_sync(int grp) {
+    asm volatile("bar.sync %0, 256;" ::"r"(grp + 1) : "memory");
+}
+
+// Sums (or, second value with MAX2, maxima) of U pairs of values over the
+// group, in the order of block_sum / block_max; pair u valid in lane 0 of the
+// group's warp u.
+template <int U, bool TWO, bool MAX2>
+__device__ __forceinline__ void group_pairs(double* a, double* b, double* sh, int grp) {
+    const int t = threadIdx.x & 255, lane = t & 31, wid = t >> 5;
+    auto add2 = [](double x, double y) { return MAX2 ? nanmax(x, y) : x + y; };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            a[u] += __shfl_down_sync(0xffffffffu, a[u], o);
+            if (TWO) b[u] = add2(b[u], __shfl_down_sync(0xffffffffu, b[u], o));
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            sh[u * 16 + wid] = a[u];
+            if (TWO) sh[u * 16 + 8 + wid] = b[u];
+        }
+    group_sync(grp);
+    if (wid < U) {
+        double x = lane < 8 ? sh[wid * 16 + lane] : 0.0;
+        double y = TWO && lane < 8 ? sh[wid * 16 + 8 + lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) {
+            x += __shfl_down_sync(0xffffffffu, x, o);
+            if (TWO) y = add2(y, __shfl_down_sync(0xffffffffu, y, o));
+        }
+        a[0] = x;
+        if (TWO) b[0] = y;
+    }
+    group_sync(grp);
+}
+
+// The partials of every slab folded in rank order, by every block for itself;
+// the result in thread 0.  which: the first of the sum's two slots.  The
+// groups take one value of one slab each (all in one group, one after another,
+// the folds took longer than the barriers).
+template <bool TWO, bool MAX2>
+__device__ __forceinline__ void group_fold(const Group& G, int which, bool apply, double* sh,
+                                           double& A, double& B) {
+    const int grp = threadIdx.x >> 8, t = threadIdx.x & 255, lane = t & 31, wid = t >> 5;
+    double* ws = sh + grp * 8;       // this group's warp sums
+    double* val = sh + 8 * kGroups;  // the values, slab by slab
+    const int n = G.R * (TWO ? 2 : 1);
+    for (int c = grp; c < n; c += kGroups) {
+        const int r = TWO ? c >> 1 : c, second = TWO ? c & 1 : 0;
+        const bool mx = MAX2 && second;
+        const int nv = apply ? G.s[r].ab : G.s[r].nb;
+        const double* pa = G.s[r].part + (which + second) * kGroupParts;
+        double x = 0.0;
+#pragma unroll 4
+        for (int q = t; q < nv; q += 256) {
+            const double y = __ldcg(pa + q);
+            x = mx ? nanmax(x, y) : x + y;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_down_sync(0xffffffffu, x, o);
+            x = mx ? nanmax(x, y) : x + y;
+        }
+        if (lane == 0) ws[wid] = x;
+        group_sync(grp);
+        if (wid == 0) {
+            x = lane < 8 ? ws[lane] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) {
+                const double y = __shfl_down_sync(0xffffffffu, x, o);
+                x = mx ? nanmax(x, y) : x + y;
+            }
+            if (lane == 0) val[c] = x;
+        }
+        group_sync(grp);
+    }
+    __syncthreads();
+    A = B = 0.0;
+    if (threadIdx.x == 0)
+        for (int r = 0; r < G.R; ++r) {
+            A += val[TWO ? 2 * r : r];
+            if (TWO) B = MAX2 ? nanmax(B, val[2 * r + 1]) : B + val[2 * r + 1];
+        }
+}
+
+// A x at (j, k) of plane i of slab s: `at(slab, offset)` is the operand.
+template <class At>
+__device__ __forceinline__ double group_stencil(const Group& G, const GroupSlab& s,
+                                                const GroupSlab& sl, const GroupSlab& sr, int i,
+                                                int j, int k, At at, double& ctr) {
+    const int ny = G.ny, nz = G.nz, h = G.h;
+    const int plane = ny * nz, p = (h + i) * plane, c = j * nz + k;
+    ctr = at(s, p + c);
+    // (the slab is chosen before the loads: in a branch of its own each
+    // operand would be waited for before the next is asked for)
+    const GroupSlab& bm = i ? s : sl;
+    const GroupSlab& bp = i + 1 < s.nxl ? s : sr;
+    const double xm = at(bm, (i ? p - plane : (h + sl.nxl - 1) * plane) + c);
+    const double xp = at(bp, (i + 1 < s.nxl ? p + plane : h * plane) + c);
+    const double ym = at(s, p + wrap(j - 1, ny) * nz + k);
+    const double yp = at(s, p + wrap(j + 1, ny) * nz + k);
+    const double zm = at(s, p + j * nz + wrap(k - 1, nz));
+    const double zp = at(s, p + j * nz + wrap(k + 1, nz));
+    double o = 0.0;
+    o += xm * G.cf.c[0][0];
+    o += ctr * G.cf.c[0][1];
+    o += xp * G.cf.c[0][2];
+    o += ym * G.cf.c[1][0];
+    o += ctr * G.cf.c[1][1];
+    o += yp * G.cf.c[1][2];
+    o += zm * G.cf.c[2][0];
+    o += ctr * G.cf.c[2][1];
+    o += zp * G.cf.c[2][2];
+    return o;
+}
+
+// One operator phase: the operand is `at(slab, q)`; `put(slab, q, centre,
+// A operand, sum a, sum b)` consumes a cell.  A block takes a run of virtual
+// blocks; where each is one tile (up to 1184 tiles per slab) the run goes
+// through the planes of a tile column, so its groups work on neighbouring
+// planes and find each other's operands in the SM's L1.
+template <bool TWO, class At, class Put>
+__device__ __forceinline__ void group_apply(const Group& G, int which, double* sh, At at, Put put) {
+    const int grp = threadIdx.x >> 8, wid = (threadIdx.x & 255) >> 5, tx = threadIdx.x & 31;
+    const int tz = (G.nz + 31) / 32, ty = (G.ny + 7) / 8, plane = G.ny * G.nz;
+    const int per = (G.nab + gridDim.x - 1) / gridDim.x;
+    const int end = min(G.nab, (int)(blockIdx.x + 1) * per);
+    for (int v = blockIdx.x * per + grp; v < end; v += kGroups) {
+        int r = 0, vb = v;
+        while (vb >= G.s[r].ab) vb -= G.s[r++].ab;
+        const GroupSlab& s = G.s[r];
+        const GroupSlab& sl = G.s[r ? r - 1 : G.R - 1];
+        const GroupSlab& sr = G.s[r + 1 < G.R ? r + 1 : 0];
+        if (G.one) {
+            const int col = vb / s.nxl;
+            vb = (vb - col * s.nxl) * (tz * ty) + col;
+        }
+        double a = 0.0, b = 0.0;
+        const int ntiles = tz * ty * s.nxl;
+        for (int t = vb; t < ntiles; t += s.ab) {
+            const int t1 = t / tz, i = t1 / ty;
+            const int k = (t - t1 * tz) * 32 + tx, j = (t1 - i * ty) * 8 + wid;
+            if (k >= G.nz || j >= G.ny) continue;
+            double c;
+            const double o = group_stencil(G, s, sl, sr, i, j, k, at, c);
+            put(s, (G.h + i) * plane + j * G.nz + k, c, o, a, b);
+        }
+        group_pairs<1, TWO, false>(&a, &b, sh + 80 + grp * 16, grp);
+        if ((threadIdx.x & 255) == 0) {
+            s.part[which * kGroupParts + vb] = a;
+            if (TWO) s.part[(which + 1) * kGroupParts + vb] = b;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBlock * kGroups, 1)
+slab_group_solve(const __grid_constant__ Group G, int first) {
+    __shared__ double sh[80 + kGroups * 16];  // folds: 32 warp sums, 48 values; then the pairs
+    // the scalars of the solve, kept (the same) by every block in shared memory
+    __shared__ SlabScalars S;
+    const int grp = threadIdx.x >> 8, tid = threadIdx.x & 255;
+    unsigned round = 0;
+    if (threadIdx.x == 0) {
+        S = *G.s[0].sc;
+        if (first) {
+            // max_res0 (src/solver/pressure.py:213) and rho1 of iteration 1
+            double a = 0.0, b = 0.0;
+            for (int r = 0; r < G.R; ++r) { a += G.s[r].send[0]; b = nanmax(b, G.s[r].send[1]); }
+            S.rho1 = a;
+            S.max_res0 = b;
+        }
+    }
+    __syncthreads();
+    const int plane = G.ny * G.nz;
+    // pointwise phases: f(slab, virtual block, first cell, end, step) in the
+    // phase kernels' distribution
+    auto pointwise = [&](auto f) {
+        for (int v = blockIdx.x + grp * gridDim.x; v < G.nnb; v += gridDim.x * kGroups) {
+            int r = 0, vb = v;
+            while (vb >= G.s[r].nb) vb -= G.s[r++].nb;
+            const GroupSlab& s = G.s[r];
+            f(s, vb, G.h * plane + vb * kBlock + tid, (G.h + s.nxl) * plane, s.nb * kBlock);
+        }
+    };
+    constexpr int B = 2;  // cells loaded before any is stored
+    double x0, x1;
+    for (int it = 0; it < kGroupIters && !S.done; ++it) {
+        const int o = S.iter & 1, n = o ^ 1;
+        {
+            const double omega = S.omega, beta = S.alpha * S.rho1 / (S.rho2 * omega);
+            group_apply<false>(
+                G, 0, sh,
+                [&](const GroupSlab& s, int q) {
+                    double p = fma(-omega, s.vv[o][q], s.pp[o][q]);
+                    p = p * beta;
+                    return p + s.res[q];
+                },
+                [&](const GroupSlab& s, int q, double c, double v, double& a, double&) {
+                    s.pp[n][q] = c;
+                    s.vv[n][q] = v;
+                    a += v * s.res0[q];
+                });
+        }
+        if (!grid_meet(G.bar, ++round)) return;
+        group_fold<false, false>(G, 0, true, sh, x0, x1);
+        if (threadIdx.x == 0) {
+            // gamma == 0 leaves the loop before DP changes
+            if (x0 == 0.0) { S.done = 1; S.status = PF_BREAKDOWN; }
+            else S.alpha = S.rho1 / x0;
+        }
+        __syncthreads();
+        if (S.done) break;
+        const double alpha = S.alpha;
+        group_apply<true>(
+            G, 1, sh, [&](const GroupSlab& s, int q) { return fma(-alpha, s.vv[n][q], s.res[q]); },
+            [&](const GroupSlab& s, int q, double c, double v, double& a, double& b) {
+                s.vv[o][q] = v;  // t
+                a += c * v;
+                b += v * v;
+            });
+        grid_arrive(G.bar);
+        // while the barrier is under way: DP += alpha pp', of cells that only
+        // this thread touches (also where (t, t) == 0 ends the solve)
+        pointwise([&](const GroupSlab& s, int, int q0, int end, int step) {
+            for (; q0 < end; q0 += B * step) {
+                double p[B], d[B];
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int q = q0 + m * step;
+                    if (q >= end) break;
+                    p[m] = s.pp[n][q]; d[m] = s.DP[q];
+                }
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int q = q0 + m * step;
+                    if (q >= end) break;
+                    s.DP[q] = fma(alpha, p[m], d[m]);
+                }
+            }
+        });
+        if (!grid_wait(G.bar, ++round)) return;
+        group_fold<true, false>(G, 1, true, sh, x0, x1);
+        if (threadIdx.x == 0) {
+            // (t, t) == 0 leaves after DP += alpha pp
+            if (x1 == 0.0) { S.done = 1; S.status = PF_BREAKDOWN; }
+            else S.omega = x0 / x1;
+        }
+        __syncthreads();
+        if (S.done) break;
+        const double omega = S.omega;
+        pointwise([&](const GroupSlab& s, int vb, int q0, int end, int step) {
+            double a = 0.0, b = 0.0;
+            for (; q0 < end; q0 += B * step) {
+                double d[B], vv[B], rs[B], t[B], r0[B];
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int q = q0 + m * step;
+                    if (q >= end) break;
+                    vv[m] = s.vv[n][q]; rs[m] = s.res[q]; t[m] = s.vv[o][q];
+                    r0[m] = s.res0[q]; d[m] = s.DP[q];
+                }
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int q = q0 + m * step;
+                    if (q >= end) break;
+                    const double sv = fma(-alpha, vv[m], rs[m]);
+                    const double rn = fma(-omega, t[m], sv);
+                    s.res[q] = rn;
+                    s.DP[q] = fma(omega, sv, d[m]);
+                    a += rn * r0[m];
+                    b = nanmax(b, fabs(rn));
+                }
+            }
+            group_pairs<1, true, true>(&a, &b, sh + 80 + grp * 16, grp);
+            if (tid == 0) {
+                s.part[3 * kGroupParts + vb] = a;
+                s.part[4 * kGroupParts + vb] = b;
+            }
+        });
+        if (!grid_meet(G.bar, ++round)) return;
+        group_fold<true, true>(G, 3, false, sh, x0, x1);
+        if (threadIdx.x == 0) {
+            // end of the iteration (src/solver/pressure.py:276-289)
+            S.rho2 = S.rho1;
+            S.rho1 = x0;
+            const double mr = x1 / S.max_res0;
+            S.max_res = mr;
+            S.iter += 1;
+            if (!(mr == mr)) { S.done = 1; S.status = PF_NONFINITE; }
+            else if (mr <= S.min_res) { S.done = 1; S.status = PF_OK; }
+            else if (S.iter >= S.max_it) { S.done = 1; S.status = PF_MAXIT; }
+        }
+        __syncthreads();
+    }
+    // every block holds the same scalars, and none reads the stored ones after
+    // the first barrier: one block writes them for every slab
+    if (!grid_meet(G.bar, ++round)) return;
+    if (blockIdx.x == 0 && threadIdx.x < G.R) *G.s[threadIdx.x].sc = S;
+}
+
 }  // namespace
 }  // namespace pf
 
@@ -427,6 +776,73 @@ int pf_slab_bicg_phase(const pf_grid* g, int halo, int phase, const double* recv
             break;
     }
     return rc_of(cudaGetLastError());
+}
+
+int pf_slab_local_solve(int count, const pf_grid* g, int halo, double rho, double dt,
+                        double min_res, int max_it, const double* const* div, double* const* DP,
+                        void* const* ws, const size_t* ws_bytes, double* const* send,
+                        void* stream, pf_solve_info* info) {
+    if (count < 1 || !g || !div || !DP || !ws || !ws_bytes || !send || !info) return PF_ERR_BAD_ARG;
+    if (count > kGroupMax || prof_on()) return PF_ERR_TOO_LARGE;
+    cudaStream_t st = (cudaStream_t)stream;
+    Group G;
+    G.R = count;
+    G.h = halo;
+    G.nab = G.nnb = 0;
+    G.one = 1;
+    for (int r = 0; r < count; ++r) {
+        if (!slab_ok(&g[r], halo) || g[r].ny != g[0].ny || g[r].nz != g[0].nz || !ws[r] ||
+            ((uintptr_t)ws[r] & 255) || ws_bytes[r] < slab_ws_bytes(&g[r]))
+            return PF_ERR_BAD_ARG;
+        const Slab sl = make_slab(&g[r], halo);
+        const SlabWs w = carve_slab(&g[r], ws[r]);
+        GroupSlab& q = G.s[r];
+        q.nxl = g[r].nx - 2 * halo;
+        q.ab = apply_blocks(sl);
+        q.nb = pointwise_blocks(sl.nint);
+        if (std::max(q.ab, q.nb) > kGroupParts || sl.d.n >= (1LL << 30)) return PF_ERR_TOO_LARGE;
+        q.res = w.v.res; q.res0 = w.v.res0;
+        q.pp[0] = w.v.pp; q.pp[1] = w.v.s;
+        q.vv[0] = w.v.vv; q.vv[1] = w.v.t;
+        q.DP = DP[r]; q.part = w.part; q.send = send[r]; q.sc = w.sc;
+        if ((long long)((g[r].nz + 31) / 32) * ((g[r].ny + 7) / 8) * q.nxl != q.ab) G.one = 0;
+        G.nab += q.ab;
+        G.nnb += q.nb;
+    }
+    G.ny = g[0].ny; G.nz = g[0].nz;
+    G.cf = lap_coef<double>(&g[0]);
+    G.bar = (unsigned*)((char*)G.s[0].sc + 128);
+    static_assert(sizeof(SlabScalars) <= 128, "the barrier words lie behind the scalars");
+    int per = 0, coop = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, slab_group_solve, kBlock * kGroups, 0) != cudaSuccess)
+        return PF_ERR_CUDA;
+    if (!coop || per < 1) return PF_ERR_TOO_LARGE;
+    for (int r = 0; r < count; ++r) {
+        const int rc = pf_slab_bicg_init(&g[r], halo, rho, dt, min_res, max_it, div[r], DP[r], ws[r],
+                                         ws_bytes[r], send[r], stream);
+        if (rc) return rc;
+    }
+    const int nb = std::min(num_sms(), (std::max(G.nab, G.nnb) + kGroups - 1) / kGroups);
+    struct { SlabScalars sc; char pad[128 - sizeof(SlabScalars)]; unsigned bar[kGridBarWords]; } hs;
+    for (int first = 1;; first = 0) {
+        if (cudaMemsetAsync(G.bar, 0, kGridBarWords * sizeof(unsigned), st) != cudaSuccess)
+            return PF_ERR_CUDA;
+        void* args[] = {&G, &first};
+        if (cudaLaunchCooperativeKernel((const void*)slab_group_solve, dim3(nb), dim3(kBlock * kGroups), args, 0,
+                                        st) != cudaSuccess ||
+            cudaMemcpyAsync(&hs, G.s[0].sc, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return PF_ERR_CUDA;
+        if (hs.bar[1]) return PF_ERR_CUDA;  // a barrier gave up
+        if (hs.sc.done) break;
+    }
+    info->max_res = hs.sc.max_res;
+    info->iterations = hs.sc.iter;
+    info->outer = 1;
+    info->status = hs.sc.status;
+    return PF_OK;
 }
 
 int pf_slab_bicg_info(const pf_grid* g, void* ws, double* out_dev, void* stream) {

@@ -45,6 +45,9 @@ for _name, (_args, _res) in {
         "pf_slab_bicg_init": ([_G, _I, _D, _D, _D, _I, _P, _P, _P, _S, _P, _P], _I),
         "pf_slab_bicg_phase": ([_G, _I, _I, _P, _I, _P, _P, _P, _P], _I),
         "pf_slab_bicg_info": ([_G, _P, _P, _P], _I),
+        "pf_slab_local_solve": ([_I, _G, _I, _D, _D, _D, _I, ctypes.POINTER(_P),
+                                 ctypes.POINTER(_P), ctypes.POINTER(_P), ctypes.POINTER(_S),
+                                 ctypes.POINTER(_P), _P, ctypes.POINTER(L.SolveInfo)], _I),
         "pf_slab_add": ([_G, _I, _P, _P, _P], _I)}.items():
     _fn = getattr(_lib, _name)
     _fn.argtypes = _args
@@ -228,6 +231,10 @@ class SlabDomain:
     def solve(self):
         """solver_bicgstab.solve over the slabs: DP from the divergence held
         in ``div``; returns a SolveInfo (max_res, iterations, status)."""
+        if isinstance(self.T, LocalSlabs):
+            info = self._solve_local()
+            if info is not None:
+                return info
         st = _P(torch.cuda.current_stream().cuda_stream)
         for s in self.slabs:
             L.check("pf_slab_bicg_init", _lib.pf_slab_bicg_init(
@@ -257,6 +264,21 @@ class SlabDomain:
                     break
         info = L.SolveInfo()
         info.max_res, info.iterations, info.outer, info.status = max_res, int(iters), 1, int(status)
+        return info
+
+    def _solve_local(self):
+        """The same solve with every slab in this process, in one library
+        call; None where that does not apply (the phases then run)."""
+        n = len(self.slabs)
+        arr = lambda name: (_P * n)(*(getattr(s, name).data_ptr() for s in self.slabs))  # noqa: E731
+        info = L.SolveInfo()
+        rc = _lib.pf_slab_local_solve(
+            n, (L.Grid * n)(*(s.grid for s in self.slabs)), HALO, self.rho, self.dt, self.min_res,
+            self.max_it, arr("div"), arr("DP"), arr("ws"),
+            (_S * n)(*(s.ws.numel() for s in self.slabs)), arr("send"), _P(torch.cuda.current_stream().cuda_stream), ctypes.byref(info))
+        if rc == L.PF_ERR_TOO_LARGE:
+            return None
+        L.check("pf_slab_local_solve", rc)
         return info
 
     def forward_step(self):

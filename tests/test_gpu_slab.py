@@ -135,3 +135,27 @@ def test_slab_restart_round_trip(tmp_path):
     for s in E.slabs:
         for name, a in zip(("u", "v", "w", "p"), f):
             assert torch.equal(getattr(s, name), extend(a, s.x0, s.nxl))
+
+
+@pytest.mark.parametrize("R,shape", [(1, (16, 12, 16)), (2, (24, 16, 20)), (3, (26, 9, 35)),
+                                     (5, (23, 6, 64)), (2, (96, 64, 64)), (24, (96, 5, 3))])
+@pytest.mark.parametrize("max_it", [5000, 7])
+def test_slab_local_solve_is_the_phases(R, shape, max_it):
+    """Every slab in one cooperative launch gives bitwise the DP, iteration
+    count, residual and status of the phase loop (ragged splits, odd extents,
+    more tiles than blocks, the iteration limit)."""
+    from pyflow_b200.slab import LocalSlabs, SlabDomain
+    sp = tuple(2 * np.pi / n for n in shape)
+    f0 = _fields(shape, seed=21)
+
+    out = []
+    for local in (True, False):
+        D = SlabDomain(shape, sp, 0.01, 1.0, 0.005, LocalSlabs(R), min_res=1e-10, max_it=max_it,
+                       poll=1)
+        if not local:
+            D._solve_local = lambda: None
+        D.set_state(*f0)
+        info = D.forward_step()
+        out.append((D.gather("DP"), D.gather("u"), info.iterations, info.max_res, info.status))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert out[0][2:] == out[1][2:]
