@@ -38,6 +38,7 @@
 #include <cstring>
 
 #include "pf_common.cuh"
+#include "pf_gridbar.cuh"
 #include "pf_kernels.cuh"
 #include "pf_sweep.cuh"
 #include "pf_grad.cuh"
@@ -93,6 +94,9 @@ bicg_init(Dims d, BicgScalars* sc, double* part, const double* src, double c1,
             sc->max_res0 = mx; sc->max_res = 0.0; sc->k = 0; sc->iter = 0;
             sc->done = 0; sc->status = PF_OK; sc->max_it = max_it;
             sc->min_res = min_res; sc->counter = 0u;
+            // the words of the one-launch solve's grid barrier
+            unsigned* bar = (unsigned*)((char*)sc + 192);
+            bar[0] = bar[1] = 0u;
         }
     }
 }
@@ -282,6 +286,485 @@ bicg_b(Dims d, Tiling tl, LapCoef<T> cf, BicgScalars* sc, double* part,
             sc->counter = 0u;
         }
     }
+}
+
+// ------------------------------------------------- the solve in one launch
+// The FP64 iterations of a grid of up to 296 tiles (two per SM) as one
+// cooperative launch: kernels CA and B over the same tiles and sums, separated
+// by grid barriers (pf_gridbar.cuh) instead of launches.  Per iteration, launch
+// pairs -> this kernel, on one B200: 24^3 28.6 -> 12.7 us, 64^3 28.3 -> 12.0,
+// 70x90x50 31.7 -> 17.0, 96^3 38.8 -> 27.8.  The pairs spent it on launch gaps,
+// the serial last block that finished each reduction, and one L2 round trip
+// per plane; left is latency: two barriers (1.6 us each at 128 blocks, 3 us at
+// 288), the ring cells' loads, and at 96^3 instruction issue.  Every block
+// folds the partials itself, in the order the last block used, one value per
+// warp, and all hold the same scalars.  The iterates are bitwise those of the
+// two kernels.  Deeper tiles (128^3: 68.4 us) stay with the launch pairs.
+
+// Sums of V values over the block in block_sum's order (the value in bit v of
+// MAXES: the maximum, NaN propagating), stored to out[v * kIterParts].
+constexpr int kIterParts = 512;     // partial slots per value (at most 2 blocks per SM)
+constexpr size_t kIterBar = 192;    // the barrier words lie behind the scalars, in their 256 bytes
+static_assert(sizeof(BicgScalars) <= kIterBar, "scalar block");
+static_assert(kIterParts <= 2 * kBlock, "fold_values takes two partials per thread");
+
+// Maximum of two values whose sign bits are clear, as unsigned integers (a
+// quarter of nanmax's instructions): NaN is above infinity there, so it stays.
+__device__ __forceinline__ double absmax(double a, double b) {
+    const unsigned long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return __longlong_as_double(x > y ? x : y);
+}
+__device__ __forceinline__ double abs_bits(double a) {
+    return __longlong_as_double(__double_as_longlong(a) & 0x7fffffffffffffffLL);
+}
+
+template <int V, unsigned MAXES>
+__device__ __forceinline__ void block_values(const double (&in)[V], double* sh, double* out) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double x[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) x[v] = in[v];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const double y = __shfl_down_sync(0xffffffffu, x[v], o);
+            x[v] = (MAXES >> v) & 1u ? absmax(x[v], y) : x[v] + y;
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int v = 0; v < V; ++v) sh[v * 8 + wid] = x[v];
+    __syncthreads();
+    if (wid < V) {
+        const bool mx = (MAXES >> wid) & 1u;
+        double y = lane < kBlock / 32 ? sh[wid * 8 + lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) {
+            const double z = __shfl_down_sync(0xffffffffu, y, o);
+            y = mx ? absmax(y, z) : y + z;
+        }
+        if (lane == 0) out[wid * kIterParts] = y;
+    }
+}
+
+// The blocks' partials of V values in finish's order, one value per warp; the
+// results in sh[0 .. V-1] for all threads.
+template <int V, unsigned MAXES>
+__device__ __forceinline__ void fold_values(const double* part, double* sh) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    constexpr int W = kBlock / 32;
+    if (wid < V) {
+        const bool mx = (MAXES >> wid) & 1u;
+        const double* pv = part + wid * kIterParts;
+        // every load before the first sum (one after another each waits for L2)
+        double x[W], y2[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const int b = 32 * w + lane;
+            x[w] = b < (int)gridDim.x ? __ldcg(pv + b) : 0.0;
+            y2[w] = b + kBlock < (int)gridDim.x ? __ldcg(pv + b + kBlock) : 0.0;
+        }
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const double y = 0.0 + x[w];
+            x[w] = 32 * w + lane + kBlock < (int)gridDim.x
+                       ? (mx ? absmax(y, y2[w]) : y + y2[w]) : y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const double y = __shfl_down_sync(0xffffffffu, x[w], o);
+                x[w] = mx ? absmax(x[w], y) : x[w] + y;
+            }
+        // the tree over the W warp sums
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int w = 0; w < o; ++w) x[w] = mx ? absmax(x[w], x[w + o]) : x[w] + x[w + o];
+        if (lane == 0) sh[wid] = x[0];
+    }
+    __syncthreads();
+}
+
+// The scalars after kernel CA of iteration k + 1 (its sums gamma, max|res|) and
+// after kernel B (its four sums), as the kernels' last blocks form them.
+__device__ __forceinline__ void solve_after_ca(BicgScalars& S, int k, double gamma, double mxr) {
+    bool stop = false;
+    if (k > 0) {
+        // stop tests of iteration k (src/solver/pressure.py:279-287)
+        S.iter = k;
+        const double mr = mxr / S.max_res0;
+        S.max_res = mr;
+        if (!(mr == mr) || isinf(mr)) { stop = true; S.status = PF_NONFINITE; }
+        else if (mr <= S.min_res) { stop = true; S.status = PF_OK; }
+        else if (k >= S.max_it) { stop = true; S.status = PF_MAXIT; }
+    }
+    if (!stop) {
+        S.gamma = gamma;
+        if (gamma == 0.0) { stop = true; S.status = PF_BREAKDOWN; }
+        else S.alpha = S.rho1 / gamma;
+    }
+    if (stop) S.done = 1;
+    S.k = k + 1;
+}
+
+__device__ __forceinline__ void solve_after_b(BicgScalars& S, const double* sums) {
+    S.buf1 = sums[0]; S.buf2 = sums[1];
+    if (S.buf2 == 0.0) {
+        S.done = 2;
+        S.status = PF_BREAKDOWN;
+    } else {
+        const double omega = S.buf1 / S.buf2;
+        S.omega = omega;
+        S.rho2 = S.rho1;
+        S.rho1 = sums[2] - omega * sums[3];  // (s - omega t, res0)
+    }
+}
+
+// One tile per block, its part of the solve kept on the SM for the whole of it:
+// res, pp and t in shared memory with the stencil operand and its ring of
+// neighbours, vv and x there too (up to 4 planes) or in registers.  (Spilled
+// registers are no place for it: after a barrier's acquire every reload from
+// local memory goes to L2; with 38 spilled words an iteration took 24 us.)  Only what neighbouring tiles read travels: a block publishes res, pp,
+// vv and t of its boundary cells (in the two kernels' buffer sets) and forms
+// the operand of its ring cells from its neighbours' published values.
+template <int XC, int PER>
+struct TileSolve {
+    static constexpr int kRing = 34 * 18;              // one plane of the operand
+    // all five fields in shared memory (one block of at most 6 planes per SM,
+    // or two of 4), or res, pp and t
+    static constexpr bool kAll = PER == 1 || XC <= 4;
+    static constexpr size_t bytes = ((kAll ? 5 : 3) * 512 * XC + (XC + 2) * kRing) * sizeof(double);
+    static constexpr int kBatch = PER == 1 ? 4 : 2;    // ring cells whose loads are in flight
+    static constexpr int kItems = (96 * XC + kBlock - 1) / kBlock;  // ring cells in y and z per thread
+};
+
+template <int XC, int PER>
+__global__ void __launch_bounds__(kBlock, PER)
+bicg_tile_solve(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc, double* part,
+                BicgVecs<double> v, double* xg) {
+    using TS = TileSolve<XC, PER>;
+    constexpr int PL = TS::kRing;
+    extern __shared__ __align__(16) double tsm[];
+    double* const res = tsm;                 // [plane][16][32]
+    double* const pp = tsm + 512 * XC;
+    double* const tt = tsm + 2 * 512 * XC;
+    double* const vs = tsm + 3 * 512 * XC;   // vv and x if kAll
+    double* const xs = tsm + 4 * 512 * XC;
+    double* const H = tsm + (TS::kAll ? 5 : 3) * 512 * XC;  // [plane + 1][18][34]: the operand
+    constexpr int XR = TS::kAll ? 1 : XC;
+    double vr[XR][2], xr[XR][2];             // else
+    __shared__ double sh[32];
+    __shared__ BicgScalars S;
+    int tx = threadIdx.x, ty = threadIdx.y;
+    unsigned* const bar = (unsigned*)((char*)sc + kIterBar);
+    unsigned round = 0;
+    if (tid0()) S = *sc;
+    // the tile, as in sweep()
+    const int t = blockIdx.x, tz = t % tl.ntz, rr = t / tl.ntz;
+    const int k0 = tz * 32, j0 = (rr % tl.nty) * 16, i0 = (rr / tl.nty) * tl.xc;
+    const int np = min(tl.xc, d.nx - i0), ez = min(32, d.nz - k0), ey = min(16, d.ny - j0);
+    const int plane = d.ny * d.nz;
+    // The offsets below are recomputed in every phase: kept across the loop
+    // they took the registers of the state and spilled.  fresh() hides where
+    // tx and ty come from.
+    auto fresh = [&]() { asm volatile("" : "+r"(tx), "+r"(ty)); };
+    auto row_ok = [&](int r) { return tx < ez && ty + 8 * r < ey; };
+    auto own_q = [&](int p, int r) { return (i0 + p) * plane + (j0 + ty + 8 * r) * d.nz + k0 + tx; };
+    auto own_e = [&](int p, int r) { return (p * 16 + ty + 8 * r) * 32 + tx; };
+    auto own_h = [&](int p, int r) { return (p + 1) * PL + (ty + 8 * r + 1) * 34 + tx + 1; };
+    // cells that a neighbouring tile reads
+    auto edge = [&](int p, int r) {
+        const int jl = ty + 8 * r;
+        return p == 0 || p == np - 1 || jl == 0 || jl == ey - 1 || tx == 0 || tx == ez - 1;
+    };
+    // ring cell `h` of plane h / 96: 32 below and 32 above in y, 16 and 16 in z;
+    // its place in H (0: none) and in the grid
+    auto ring = [&](int h, int& e, int& q) {
+        const int p = h / 96, c = h - p * 96;
+        e = 0;
+        if (p >= np) return;
+        int row, col;
+        if (c < 64) {
+            row = c < 32 ? 0 : ey + 1;
+            col = (c & 31) + 1;
+            if (col > ez) return;
+        } else {
+            row = ((c - 64) & 15) + 1;
+            col = c < 80 ? 0 : ez + 1;
+            if (row > ey) return;
+        }
+        e = (p + 1) * PL + row * 34 + col;
+        q = (i0 + p) * plane + wrap(j0 + row - 1, d.ny) * d.nz + wrap(k0 + col - 1, d.nz);
+    };
+    // the operand of every ring cell, op(q): first the planes beside the tile,
+    // then the rows and columns around it
+    auto fill_ring = [&](auto load, auto op) {
+        const int qm = wrap(i0 - 1, d.nx) * plane, qp = wrap(i0 + np, d.nx) * plane;
+        // (at most four cells' values at a time)
+#pragma unroll
+        for (int m0 = 0; m0 < 4; m0 += TS::kBatch) {
+            decltype(load(0)) w[TS::kBatch];
+#pragma unroll
+            for (int m = m0; m < m0 + TS::kBatch; ++m)
+                if (row_ok(m & 1))
+                    w[m - m0] = load((m < 2 ? qm : qp) + (j0 + ty + 8 * (m & 1)) * d.nz + k0 + tx);
+#pragma unroll
+            for (int m = m0; m < m0 + TS::kBatch; ++m)
+                if (row_ok(m & 1)) H[own_h(m < 2 ? -1 : np, m & 1)] = op(w[m - m0]);
+            fresh();
+        }
+#pragma unroll
+        for (int m0 = 0; m0 < TS::kItems; m0 += TS::kBatch) {
+            decltype(load(0)) w[TS::kBatch];
+            int e[TS::kBatch];
+#pragma unroll
+            for (int m = 0; m < TS::kBatch; ++m) {
+                int q;
+                ring(ty * 32 + tx + (m0 + m) * kBlock, e[m], q);
+                if (e[m]) w[m] = load(q);
+            }
+#pragma unroll
+            for (int m = 0; m < TS::kBatch; ++m)
+                if (e[m]) H[e[m]] = op(w[m]);
+            fresh();
+        }
+    };
+    auto stencil = [&](int h) {
+        const double c = H[h];
+        double b = 0.0;
+        b += H[h - PL] * cf.c[0][0];
+        b += c * cf.c[0][1];
+        b += H[h + PL] * cf.c[0][2];
+        b += H[h - 34] * cf.c[1][0];
+        b += c * cf.c[1][1];
+        b += H[h + 34] * cf.c[1][2];
+        b += H[h - 1] * cf.c[2][0];
+        b += c * cf.c[2][1];
+        b += H[h + 1] * cf.c[2][2];
+        return b;
+    };
+    // a barrier that gave up ends the solve with an error
+    auto failed = [&]() {
+        if (tid0()) { sc->status = PF_ERR_CUDA; sc->done = 1; }
+    };
+    // bicg_init's state (buffer set 1): res = b, pp = vv = t = x = 0
+    auto VV = [&](int p, int r) -> double& {
+        if constexpr (TS::kAll) return vs[own_e(p, r)]; else return vr[p][r];
+    };
+    auto X = [&](int p, int r) -> double& {
+        if constexpr (TS::kAll) return xs[own_e(p, r)]; else return xr[p][r];
+    };
+    // f(plane, row) for the thread's cells, one plane after another (the
+    // compiler may not mix the planes: their loads would fill the registers)
+    auto cells = [&](auto f) {
+#pragma unroll
+        for (int p = 0; p < XC; ++p) {
+            if (PER > 1) asm volatile("" ::: "memory");
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                if (p < np && row_ok(r)) f(p, r);
+        }
+    };
+    // the same with res0 of the cell: held in registers by a block that has the
+    // SM to itself, else loaded a plane ahead
+    double r0s[PER == 1 ? XC : 1][2];
+    auto cells_r0 = [&](auto f) {
+        double nx[2];
+        auto fetch = [&](int p) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if constexpr (PER == 1) nx[r] = r0s[p][r];
+                else nx[r] = p < np && row_ok(r) ? __ldg(v.res0 + own_q(p, r)) : 0.0;
+            }
+        };
+        fetch(0);
+#pragma unroll
+        for (int p = 0; p < XC; ++p) {
+            const double r0[2] = {nx[0], nx[1]};
+            if (p + 1 < XC) fetch(p + 1);
+            if (PER > 1) asm volatile("" ::: "memory");
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                if (p < np && row_ok(r)) f(p, r, r0[r]);
+        }
+    };
+    if constexpr (!TS::kAll) {
+#pragma unroll
+        for (int p = 0; p < XR; ++p)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) vr[p][r] = xr[p][r] = 0.0;
+    }
+    cells([&](int p, int r) {
+        const int e = own_e(p, r);
+        const double b = v.res0[own_q(p, r)];
+        res[e] = b;
+        if constexpr (PER == 1) r0s[p][r] = b;
+        pp[e] = tt[e] = 0.0;
+        if constexpr (TS::kAll) vs[e] = xs[e] = 0.0;
+    });
+    __syncthreads();
+    while (!S.done) {
+        fresh();
+        const int k = S.k;
+        const bool odd = k & 1, fin = k > 0;  // CA(k) writes set k&1 and reads the other
+        double val[4] = {0.0, 0.0, 0.0, 0.0};
+        {
+            const double alpha = S.alpha, omega = S.omega;
+            const double beta = (S.alpha * S.rho1) / (S.rho2 * S.omega);
+            const double* ro = odd ? v.res[0] : v.res[1];
+            const double* po = odd ? v.pp[0] : v.pp[1];
+            const double* vo = odd ? v.vv[0] : v.vv[1];
+            double* rn = odd ? v.res[1] : v.res[0];
+            double* pn = odd ? v.pp[1] : v.pp[0];
+            double* vn = odd ? v.vv[1] : v.vv[0];
+            cells([&](int p, int r) {
+                    const int e = own_e(p, r);
+                    double rv = res[e];
+                    const double pv = pp[e];
+                    if (fin) {
+                        const double s = fma(-alpha, VV(p, r), rv);
+                        rv = fma(-omega, tt[own_e(p, r)], s);
+                        X(p, r) = fma(omega, s, fma(alpha, pv, X(p, r)));
+                        res[e] = rv;
+                    }
+                    double q = fma(-omega, VV(p, r), pv);
+                    q = q * beta;
+                    q = q + rv;
+                    pp[e] = q;
+                    H[own_h(p, r)] = q;
+                    val[1] = absmax(val[1], abs_bits(rv));
+                    if (edge(p, r)) { rn[own_q(p, r)] = rv; pn[own_q(p, r)] = q; }
+            });
+            struct Raw { double r, p, v, t; };
+            fresh();
+            fill_ring([&](int q) { return Raw{ro[q], po[q], vo[q], v.t[q]}; },
+                      [&](const Raw& a) {
+                          double rv = a.r;
+                          if (fin) rv = fma(-omega, a.t, fma(-alpha, a.v, a.r));
+                          double q = fma(-omega, a.v, a.p);
+                          q = q * beta;
+                          return q + rv;
+                      });
+            __syncthreads();
+            fresh();
+            cells_r0([&](int p, int r, double r0) {
+                    const double b = stencil(own_h(p, r));
+                    VV(p, r) = b;
+                    val[0] += b * r0;
+                    if (edge(p, r)) vn[own_q(p, r)] = b;
+            });
+        }
+        const double v2[2] = {val[0], val[1]};
+        block_values<2, 2u>(v2, sh, part + blockIdx.x);
+        if (!grid_meet(bar, ++round)) return failed();
+        fold_values<2, 2u>(part, sh);
+        if (tid0()) solve_after_ca(S, k, sh[0], sh[1]);
+        __syncthreads();
+        if (S.done) break;
+        {
+            fresh();
+            const double alpha = S.alpha;
+            const double* rn = odd ? v.res[1] : v.res[0];
+            const double* vn = odd ? v.vv[1] : v.vv[0];
+            cells([&](int p, int r) { H[own_h(p, r)] = fma(-alpha, VV(p, r), res[own_e(p, r)]); });
+            fresh();
+            fill_ring([&](int q) { return make_double2(rn[q], vn[q]); },
+                      [&](const double2& a) { return fma(-alpha, a.y, a.x); });
+            __syncthreads();
+            val[0] = val[1] = 0.0;
+            fresh();
+            cells_r0([&](int p, int r, double r0) {
+                    const int h = own_h(p, r);
+                    const double c = H[h], b = stencil(h);
+                    tt[own_e(p, r)] = b;
+                    if (edge(p, r)) v.t[own_q(p, r)] = b;
+                    val[0] += c * b;
+                    val[1] += b * b;
+                    val[2] += c * r0;
+                    val[3] += b * r0;
+            });
+        }
+        block_values<4, 0u>(val, sh, part + 2 * kIterParts + blockIdx.x);
+        if (!grid_meet(bar, ++round)) return failed();
+        fold_values<4, 0u>(part + 2 * kIterParts, sh);
+        if (tid0()) solve_after_b(S, sh);
+        __syncthreads();
+        if (S.done == 2) {
+            // (t,t) == 0 breakdown: the reference has applied DP += alpha pp and
+            // stops (src/solver/pressure.py:251,266-267)
+            cells([&](int p, int r) { X(p, r) = fma(S.alpha, pp[own_e(p, r)], X(p, r)); });
+        }
+    }
+    cells([&](int p, int r) { xg[own_q(p, r)] = X(p, r); });
+    // every block holds the same scalars: once all have read the stored ones,
+    // one block stores them
+    if (!grid_meet(bar, ++round)) return failed();
+    if (blockIdx.x == 0 && tid0()) { S.done = 1; *sc = S; }
+}
+
+typedef void (*TileKernel)(Dims, Tiling, LapCoef<double>, BicgScalars*, double*, BicgVecs<double>,
+                           double*);
+
+constexpr int kTilePlanes = 6;  // deepest tile: two blocks' shared memory per SM
+
+template <int PER>
+static TileKernel tile_kernel_of(int xc, size_t* smem) {
+    switch (xc) {
+        case 6: *smem = TileSolve<6, PER>::bytes; return bicg_tile_solve<6, PER>;
+        case 5: *smem = TileSolve<5, PER>::bytes; return bicg_tile_solve<5, PER>;
+        default: *smem = TileSolve<4, PER>::bytes; return bicg_tile_solve<4, PER>;
+    }
+}
+
+// One block per SM, with its registers, where the tiles are that few.
+static TileKernel tile_kernel(const Tiling& tl, size_t* smem) {
+    return tl.ntiles <= num_sms() ? tile_kernel_of<1>(tl.xc, smem) : tile_kernel_of<2>(tl.xc, smem);
+}
+
+static cudaError_t tile_attributes() {
+    for (int xc = 4; xc <= kTilePlanes; ++xc)
+        for (int per = 1; per <= 2; ++per) {
+            size_t smem;
+            TileKernel k = per == 1 ? tile_kernel_of<1>(xc, &smem) : tile_kernel_of<2>(xc, &smem);
+            const cudaError_t e =
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+// True when the whole solve runs as one cooperative launch: every block has
+// one tile of at most kTilePlanes planes and all are resident at once.
+static bool tile_solve_applies(const Dims& d) {
+    const Tiling tl = make_tiling(d, 16);
+    if (tl.xc > kTilePlanes || tl.ntiles > std::min(2 * num_sms(), kIterParts) || d.n >= (1LL << 30))
+        return false;
+    if (once_per_context((const void*)&tile_attributes, &tile_attributes) != cudaSuccess) return false;
+    size_t smem;
+    TileKernel k = tile_kernel(tl, &smem);
+    int dev = 0, coop = 0, per = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kBlock, smem) == cudaSuccess &&
+           tl.ntiles <= (long long)per * num_sms();
+}
+
+static cudaError_t launch_tile_solve(const Dims& d, const LapCoef<double>& cf, BicgScalars* sc,
+                                     double* part, const BicgVecs<double>& v, double* x,
+                                     cudaStream_t s) {
+    const Tiling tl = make_tiling(d, 16);
+    cudaLaunchConfig_t cfg = {};
+    TileKernel k = tile_kernel(tl, &cfg.dynamicSmemBytes);
+    cfg.gridDim = dim3((unsigned)tl.ntiles);
+    cfg.blockDim = dim3(32, 8);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, d, tl, cf, sc, part, v, x);
 }
 
 // ------------------------------------------------ mixed-precision refinement
@@ -489,6 +972,14 @@ static int run_iterations(const Dims& d, const LapCoef<T>& cf,
     const Tiling ta = make_tiling(d, 8 * PhaseCA<T>::R);
     const Tiling tb = make_tiling(d, 8 * PhaseB<T>::R);
     const int ga = tiled_grid(ta), gb = tiled_grid(tb);
+    if constexpr (sizeof(T) == 8) {
+        // (the per-kernel timers count the two kernels)
+        if (!prof_on() && tile_solve_applies(d)) {
+            if (launch_tile_solve(d, cf, sc, part, v, x, s) != cudaSuccess) return PF_ERR_CUDA;
+            const int rc = read_scalars(sc, hs, s);
+            return rc ? rc : (hs->status == PF_ERR_CUDA ? PF_ERR_CUDA : PF_OK);
+        }
+    }
     dim3 blk2(32, 8);
     const char* nca = sizeof(T) == 8 ? "bicg_ca_f64" : "bicg_ca_f32";
     const char* nb = sizeof(T) == 8 ? "bicg_b_f64" : "bicg_b_f32";
@@ -1162,13 +1653,32 @@ static int plan_layout(const pf_grid* g, int prec, double min_res, const double*
     return PF_OK;
 }
 
+// After the solve (node `dep`): the result next to the statistics, p += DP, the
+// projection and the monitor statistics.
+static int add_step_end(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g, PlanLayout& P,
+                        double* u, double* v, double* w, double* p, double* DP, double rho,
+                        double dt, bool mixed, double* stats, cudaStream_t cs,
+                        cudaGraphNode_t* end) {
+    int rc;
+    cudaGraph_t seg = nullptr;
+    if ((rc = capture_begin(cs, nullptr))) return rc;
+    step_info<<<1, 32, 0, cs>>>(P.sc, mixed ? 1 : 0, stats + 5);
+    add_inplace<<<pointwise_grid(P.d.n), kBlock, 0, cs>>>(P.d.n, DP, p);
+    launch_vel_corr(g, DP, dt / rho, u, v, w, cs);
+    launch_stats(g, u, v, w, stats, P.R, cs);
+    if ((rc = capture_end(cs, &seg))) return rc;
+    rc = add_child(G, dep, seg, end);
+    cudaGraphDestroy(seg);
+    return rc;
+}
+
 // Adds one request's step after the predictor (node `dep`) to graph G:
 // divergence and solver set-up, the solver's WHILE loop(s), then p += DP,
 // the projection and the monitor statistics.  *end gets the last node.
 static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g, int prec,
                            PlanLayout& P, double* u, double* v, double* w, double* p,
                            double* DP, double rho, double dt, double min_res, int max_it,
-                           double* stats, cudaStream_t cs, cudaGraphNode_t* end) {
+                           double* stats, bool alone, cudaStream_t cs, cudaGraphNode_t* end) {
     const Dims d = P.d;
     BicgScalars* sc = P.sc;
     double* part = P.part;
@@ -1178,6 +1688,9 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
     max_it = std::max(max_it, 1);
     dim3 blk2(32, 8);
     int rc = PF_OK;
+    // the FP64 solve in one cooperative launch, unless it is one of several
+    // parallel branches (their blocks could wait on one another for room)
+    const bool one_launch = prec == PF_FP64 && alone && tile_solve_applies(d);
     // ---- divergence, solver set-up
     cudaGraph_t seg1 = nullptr;
     cudaGraph_t C = G;        // the graph that holds the solver's loops
@@ -1212,6 +1725,14 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
         const Tiling ta = make_tiling(d, 8 * PhaseCA<double>::R);
         bicg_init<double, false><<<gp, kBlock, 0, cs>>>(d, sc, part, P.div, c1, c2, P.v64, DP,
                                                        max_it, min_res);
+        if (one_launch) {
+            const cudaError_t e = launch_tile_solve(d, cf, sc, part, P.v64, DP, cs);
+            if ((rc = capture_end(cs, &seg1))) return rc;
+            if (e == cudaSuccess) rc = add_child(G, dep, seg1, &nsolved);
+            cudaGraphDestroy(seg1);
+            if (e != cudaSuccess || rc) return PF_ERR_CUDA;
+            return add_step_end(G, nsolved, g, P, u, v, w, p, DP, rho, dt, false, stats, cs, end);
+        }
         bicg_ca<double><<<tiled_grid(ta), blk2, 0, cs>>>(d, ta, cf, sc, part, P.v64, DP);
     } else {
         // the refinement starts from the previous step's DP (zero before the
@@ -1351,17 +1872,7 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
         cudaGraphDestroy(post);
         if (rc) return rc;
     }
-    // ---- p += DP, projection, statistics
-    cudaGraph_t seg3 = nullptr;
-    if ((rc = capture_begin(cs, nullptr))) return rc;
-    step_info<<<1, 32, 0, cs>>>(sc, prec != PF_FP64 ? 1 : 0, stats + 5);
-    add_inplace<<<gp, kBlock, 0, cs>>>(d.n, DP, p);
-    launch_vel_corr(g, DP, dt / rho, u, v, w, cs);
-    launch_stats(g, u, v, w, stats, P.R, cs);
-    if ((rc = capture_end(cs, &seg3))) return rc;
-    rc = add_child(G, nsolved, seg3, end);
-    cudaGraphDestroy(seg3);
-    return rc;
+    return add_step_end(G, nsolved, g, P, u, v, w, p, DP, rho, dt, prec != PF_FP64, stats, cs, end);
 }
 
 // Captures the body of `enqueue(cs)` as a child node of G (no dependency).
@@ -1461,7 +1972,7 @@ int step_plan_create(const pf_grid* g, int prec, int rk4, double* u, double* v,
              }, &n0)))
             break;
         if ((rc = add_solve_chain(G, n0, g, prec, P, u, v, w, p, DP, rho, dt, min_res, max_it,
-                                  stats, cs, &nend)))
+                                  stats, true, cs, &nend)))
             break;
         if (cudaGraphInstantiate(&plan->exec, G, 0) != cudaSuccess) { rc = PF_ERR_CUDA; break; }
     } while (0);
@@ -1528,7 +2039,7 @@ int batch_plan_create(int prec, int rk4, const pf_batch_member* m, int count, vo
             cudaGraphNode_t nend;
             rc = add_solve_chain(G, n0, &m[r].grid, prec, P[r], m[r].u, m[r].v, m[r].w, m[r].p,
                                  m[r].DP, m[r].rho, m[r].dt, m[r].min_res, m[r].max_it,
-                                 m[r].stats, cs, &nend);
+                                 m[r].stats, false, cs, &nend);
         }
         if (rc != PF_OK) break;
         if (cudaGraphInstantiate(&plan->exec, G, 0) != cudaSuccess) { rc = PF_ERR_CUDA; break; }
