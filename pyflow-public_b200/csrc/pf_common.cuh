@@ -68,6 +68,16 @@ __device__ inline double nanmax(double a, double b) {
     return (a != a || b != b) ? __longlong_as_double(0x7ff8000000000000LL) : fmax(a, b);
 }
 
+// Maximum of two values whose sign bits are clear, as unsigned integers (a
+// quarter of nanmax's instructions): NaN is above infinity there, so it stays.
+__device__ __forceinline__ double absmax(double a, double b) {
+    const unsigned long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return __longlong_as_double(x > y ? x : y);
+}
+__device__ __forceinline__ double abs_bits(double a) {
+    return __longlong_as_double(__double_as_longlong(a) & 0x7fffffffffffffffLL);
+}
+
 // block-wide max of non-negative values; a NaN anywhere gives NaN
 template <int NT>
 __device__ inline double block_max(double v, double* sh) {

@@ -308,16 +308,6 @@ constexpr size_t kIterBar = 192;    // the barrier words lie behind the scalars,
 static_assert(sizeof(BicgScalars) <= kIterBar, "scalar block");
 static_assert(kIterParts <= 2 * kBlock, "fold_values takes two partials per thread");
 
-// Maximum of two values whose sign bits are clear, as unsigned integers (a
-// quarter of nanmax's instructions): NaN is above infinity there, so it stays.
-__device__ __forceinline__ double absmax(double a, double b) {
-    const unsigned long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-    return __longlong_as_double(x > y ? x : y);
-}
-__device__ __forceinline__ double abs_bits(double a) {
-    return __longlong_as_double(__double_as_longlong(a) & 0x7fffffffffffffffLL);
-}
-
 template <int V, unsigned MAXES>
 __device__ __forceinline__ void block_values(const double (&in)[V], double* sh, double* out) {
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -844,58 +834,253 @@ mixed_residual(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc,
     }
 }
 
-// The direct solve's check: max|b| and max|b - A x| in one sweep, b = (src
-// c1) c2 formed on the fly (16 bytes per cell); nothing is stored.
-struct PhaseCheck {
-    static constexpr int R = 4;
-    const double *x, *src;
-    double c1, c2, mx, mb;
-    struct Raw { double x; };
-    struct Ext { double s; };
-    __device__ Raw raw(long long q, int = 0, int = 0, int = 0) const { return Raw{x[q]}; }
-    __device__ Ext ext(long long q) const { return Ext{src[q]}; }
-    __device__ double op(const Raw& a) const { return a.x; }
-    __device__ void epi(long long, double, double ax, const Raw&, const Ext& e) {
-        const double b = (e.s * c1) * c2;
-        mx = nanmax(mx, fabs(b - ax));
-        mb = nanmax(mb, fabs(b));
+// One reduction of V values over the grid, finished by the last block to
+// arrive: every block stores its V sums (or, bit v of MAXES, integer maxima of
+// non-negative values) at part[v * stride + block]; the last block's folds go
+// to res (shared memory), true there.  One barrier per level for all values
+// together: value by value, the two levels took 8 us of an 11 us kernel.
+template <int V, unsigned MAXES>
+__device__ __forceinline__ void block_reduce(double (&x)[V], double* sh, double* res) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const double y = __shfl_down_sync(0xffffffffu, x[v], o);
+            x[v] = (MAXES >> v) & 1u ? absmax(x[v], y) : x[v] + y;
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int v = 0; v < V; ++v) sh[v * 8 + wid] = x[v];
+    __syncthreads();
+    if (wid < V) {
+        const bool mx = (MAXES >> wid) & 1u;
+        double y = lane < kBlock / 32 ? sh[wid * 8 + lane] : 0.0;
+        for (int o = 4; o > 0; o >>= 1) {
+            const double z = __shfl_down_sync(0xffffffffu, y, o);
+            y = mx ? absmax(y, z) : y + z;
+        }
+        if (lane == 0) res[wid] = y;
     }
+    __syncthreads();
+}
+
+template <int V, unsigned MAXES>
+__device__ __forceinline__ bool grid_reduce(double (&x)[V], BicgScalars* sc, double* part,
+                                            int stride, double* sh, double* res) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    block_reduce<V, MAXES>(x, sh, res);
+    if (tid < V) part[tid * stride + blockIdx.x] = res[tid];
+    if (!arrive_last(sc)) return false;
+#pragma unroll
+    for (int v = 0; v < V; ++v) x[v] = 0.0;
+    for (int b0 = tid; b0 < (int)gridDim.x; b0 += 2 * kBlock) {
+        double y[V][2];
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+                y[v][m] = b0 + m * kBlock < (int)gridDim.x ? __ldcg(part + v * stride + b0 + m * kBlock) : 0.0;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int m = 0; m < 2; ++m) x[v] = (MAXES >> v) & 1u ? absmax(x[v], y[v][m]) : x[v] + y[v][m];
+    }
+    block_reduce<V, MAXES>(x, sh, res);
+    return true;
+}
+
+// Blocks of the pointwise kernels that reduce: one wave of four per SM (three
+// waves: each wave's arrivals cost a fence, 31.5 against 28.9 us at 128^3).
+constexpr int kPassBlocks = 592;
+
+// After a solve, in one pass over the grid:
+//   CHECK    max|b| and max|b - A x| of the direct solve's x = DP (b = (src c1)
+//            c2 formed on the fly), the end of the solve;
+//   CORRECT  p += DP (src/solver/pressure.py:294) and the projection u_d -=
+//            scale grad DP (src/data/domain.py:394-402).
+// With both, the correction does not wait for the check: where it then fails
+// (a source with a mean, a tolerance below the transforms' rounding),
+// project_undo takes it back before FP64 BiCGStab passes go on from DP.  80
+// bytes per cell, 26.6 us at 128^3 and 7.5 at 64^3 (6.3 TB/s of L2 and HBM at
+// 128^3); as three kernels (96 bytes) with an IF node between the check and the
+// correction it took 57 and 26 us of a step.
+// A right-hand side that is not finite (sc->nonfin) gives DP = 0, no
+// correction and PF_NONFINITE.  VEC: two cells in z per thread, 16-byte loads.
+struct ProjectArgs {
+    Dims d;
+    int tz, ty;             // tiles of a plane
+    long long ntiles;
+    LapCoef<double> cf;
+    BicgScalars* sc;
+    double* part;
+    const double* src;
+    double c1, c2, min_res;
+    int max_it;
+    double* DP;
+    double scale, dxi, dyi, dzi;
+    double *u, *v, *w, *p;
+    int use_cond;           // graph: the IF node's handle
+    cudaGraphConditionalHandle cond;
 };
 
-// Ends the direct solve: done when the true residual meets the tolerance,
-// otherwise (a source with a mean, a tolerance below its rounding) FP64
-// BiCGStab passes follow, started from x.  In a graph `cond` is the handle of
-// the IF node that holds them.
-__global__ void __launch_bounds__(kBlock, 2)
-spectral_check(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc, double* part,
-               const double* __restrict__ src, const double* __restrict__ x, double c1, double c2,
-               double min_res, int max_it, int use_cond, cudaGraphConditionalHandle cond) {
-    __shared__ double sh[32];
+template <int V>
+struct Cells {
+    double a[V];
+};
+template <int V>
+__device__ __forceinline__ Cells<V> ld_cells(const double* p) {
+    Cells<V> c;
+    if constexpr (V == 2) {
+        const double2 t = *(const double2*)p;
+        c.a[0] = t.x;
+        c.a[1] = t.y;
+    } else {
+        c.a[0] = *p;
+    }
+    return c;
+}
+template <int V>
+__device__ __forceinline__ void st_cells(double* p, const Cells<V>& c) {
+    if constexpr (V == 2) *(double2*)p = make_double2(c.a[0], c.a[1]);
+    else *p = c.a[0];
+}
+
+template <int V, bool CHECK, bool CORRECT>
+__global__ void __launch_bounds__(kBlock, 4)
+project_kernel(ProjectArgs A) {
+    __shared__ double sh[16], res[2];
     pdl_wait();
-    PhaseCheck ph{x, src, c1, c2, 0.0, 0.0};
-    sweep<double>(d, tl, cf, ph);
-    const double bm = block_max<kBlock>(ph.mx, sh);
-    const double bb = block_max<kBlock>(ph.mb, sh);
-    if (tid0()) { part[blockIdx.x] = bm; part[kMaxPartials + blockIdx.x] = bb; }
-    if (arrive_last(sc)) {
-        const double mx = finish<true>(part, sh);
-        const double mb = finish<true>(part + kMaxPartials, sh);
+    const Dims d = A.d;
+    const bool bad = CHECK && A.sc->nonfin != 0;
+    double mx = 0.0, mb = 0.0;
+    const long long plane = (long long)d.ny * d.nz;
+    for (long long t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
+        const int t1 = (int)(t / A.tz), i = t1 / A.ty;
+        const int k = ((int)(t - (long long)t1 * A.tz) * 32 + threadIdx.x) * V;
+        const int j = (t1 - i * A.ty) * 8 + threadIdx.y;
+        if (k >= d.nz || j >= d.ny) continue;
+        const long long row = i * plane + (long long)j * d.nz, q = row + k;
+        if (bad) {
+            Cells<V> z;
+#pragma unroll
+            for (int m = 0; m < V; ++m) z.a[m] = 0.0;
+            st_cells<V>(A.DP + q, z);
+            continue;
+        }
+        const Cells<V> c = ld_cells<V>(A.DP + q);
+        const Cells<V> xm = ld_cells<V>(A.DP + wrap(i - 1, d.nx) * plane + (long long)j * d.nz + k);
+        const Cells<V> ym = ld_cells<V>(A.DP + i * plane + (long long)wrap(j - 1, d.ny) * d.nz + k);
+        const double zm = A.DP[row + wrap(k - 1, d.nz)];
+        Cells<V> xp, yp, src;
+        double zp = 0.0;
+        if (CHECK) {
+            xp = ld_cells<V>(A.DP + wrap(i + 1, d.nx) * plane + (long long)j * d.nz + k);
+            yp = ld_cells<V>(A.DP + i * plane + (long long)wrap(j + 1, d.ny) * d.nz + k);
+            zp = A.DP[row + wrap(k + V, d.nz)];
+            src = ld_cells<V>(A.src + q);
+        }
+        Cells<V> u, v, w, p;
+        if (CORRECT) {
+            u = ld_cells<V>(A.u + q);
+            v = ld_cells<V>(A.v + q);
+            w = ld_cells<V>(A.w + q);
+            p = ld_cells<V>(A.p + q);
+        }
+#pragma unroll
+        for (int m = 0; m < V; ++m) {
+            const double x = c.a[m], zl = m ? c.a[m - 1] : zm;
+            if (CHECK) {
+                const double zr = m + 1 < V ? c.a[m + 1 < V ? m + 1 : m] : zp;
+                double ax = 0.0;
+                ax += xm.a[m] * A.cf.c[0][0];
+                ax += x * A.cf.c[0][1];
+                ax += xp.a[m] * A.cf.c[0][2];
+                ax += ym.a[m] * A.cf.c[1][0];
+                ax += x * A.cf.c[1][1];
+                ax += yp.a[m] * A.cf.c[1][2];
+                ax += zl * A.cf.c[2][0];
+                ax += x * A.cf.c[2][1];
+                ax += zr * A.cf.c[2][2];
+                const double b = (src.a[m] * A.c1) * A.c2;
+                mx = absmax(mx, abs_bits(b - ax));
+                mb = absmax(mb, abs_bits(b));
+            }
+            if (CORRECT) {
+                p.a[m] = p.a[m] + x;
+                u.a[m] = fma(-A.scale, (x - xm.a[m]) * A.dxi, u.a[m]);  // var.sub_(scale, grad)
+                v.a[m] = fma(-A.scale, (x - ym.a[m]) * A.dyi, v.a[m]);
+                w.a[m] = fma(-A.scale, (x - zl) * A.dzi, w.a[m]);
+            }
+        }
+        if (CORRECT) {
+            st_cells<V>(A.p + q, p);
+            st_cells<V>(A.u + q, u);
+            st_cells<V>(A.v + q, v);
+            st_cells<V>(A.w + q, w);
+        }
+    }
+    if (!CHECK) return;
+    BicgScalars* sc = A.sc;
+    double red[2] = {mx, mb};
+    if (grid_reduce<2, 3u>(red, sc, A.part, kPassBlocks, sh, res)) {
+        const double fx = res[0], fb = res[1];
         if (tid0()) {
-            const double ratio = mb == 0.0 ? 0.0 : mx / mb;
-            sc->max_b = mb; sc->scale = mx; sc->true_res = mx; sc->max_res = ratio;
+            const double nan = __longlong_as_double(0x7ff8000000000000LL);
+            const double ratio = bad ? nan : (fb == 0.0 ? 0.0 : fx / fb);
+            sc->max_b = fb; sc->scale = fx; sc->true_res = fx; sc->max_res = ratio;
             sc->outer = 1;
-            sc->total = sc->iter = mb == 0.0 ? 0 : 1;
+            sc->total = sc->iter = fb == 0.0 && !bad ? 0 : 1;
             sc->use64 = 1; sc->prev_ratio = ratio;
             bool more = false;
             if (!(ratio == ratio) || isinf(ratio)) sc->status = PF_NONFINITE;
-            else if (ratio <= min_res) sc->status = PF_OK;
-            else if (max_it <= 1) sc->status = PF_MAXIT;
+            else if (ratio <= A.min_res) sc->status = PF_OK;
+            else if (A.max_it <= 1) sc->status = PF_MAXIT;
             else more = true;
             sc->done = more ? 0 : 1;
+            sc->redo = more ? 1 : 0;
+            sc->nonfin = 0;
             sc->counter = 0u;
-            if (use_cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
+            if (A.use_cond) cudaGraphSetConditional(A.cond, more ? 1u : 0u);
         }
     }
+}
+
+// Takes project_kernel's correction back (to rounding).
+__global__ void __launch_bounds__(256)
+project_undo(Dims d, const double* __restrict__ DP, double scale, double dxi, double dyi,
+             double dzi, double* __restrict__ u, double* __restrict__ v, double* __restrict__ w,
+             double* __restrict__ p) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= d.nz || j >= d.ny) return;
+    const long long q = idx(d, i, j, k);
+    const double c = DP[q];
+    u[q] = fma(scale, (c - DP[idx(d, wrap(i - 1, d.nx), j, k)]) * dxi, u[q]);
+    v[q] = fma(scale, (c - DP[idx(d, i, wrap(j - 1, d.ny), k)]) * dyi, v[q]);
+    w[q] = fma(scale, (c - DP[idx(d, i, j, wrap(k - 1, d.nz))]) * dzi, w[q]);
+    p[q] = p[q] - c;
+}
+
+template <bool CHECK, bool CORRECT>
+static void launch_project(const char* name, const pf_grid* g, ProjectArgs A, cudaStream_t s) {
+    A.d = Dims{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    A.cf = lap_coef<double>(g);
+    A.dxi = 1.0 / g->dx; A.dyi = 1.0 / g->dy; A.dzi = 1.0 / g->dz;
+    uintptr_t bits = (uintptr_t)A.DP;
+    if (CHECK) bits |= (uintptr_t)A.src;
+    if (CORRECT) bits |= (uintptr_t)A.u | (uintptr_t)A.v | (uintptr_t)A.w | (uintptr_t)A.p;
+    const bool vec = g->nz % 2 == 0 && (bits & 15) == 0;
+    const int zt = vec ? 64 : 32;
+    A.tz = (g->nz + zt - 1) / zt;
+    A.ty = (g->ny + 7) / 8;
+    A.ntiles = (long long)A.tz * A.ty * g->nx;
+    const int blocks = (int)std::min<long long>(A.ntiles, kPassBlocks);
+    if (vec)
+        PF_LAUNCH(name, s, launch_pdl(project_kernel<2, CHECK, CORRECT>, dim3(blocks), dim3(32, 8), 0, s, A));
+    else
+        PF_LAUNCH(name, s, launch_pdl(project_kernel<1, CHECK, CORRECT>, dim3(blocks), dim3(32, 8), 0, s, A));
 }
 
 // b = (src c1) c2
@@ -904,17 +1089,6 @@ scaled_source(long long n, const double* src, double c1, double c2, double* b) {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
          q += (long long)gridDim.x * blockDim.x)
         b[q] = (src[q] * c1) * c2;
-}
-
-static void launch_spectral_check(const pf_grid* g, BicgScalars* sc, double* part,
-                                  const double* src, const double* x, double c1, double c2,
-                                  double min_res, int max_it, cudaStream_t s, int use_cond = 0,
-                                  cudaGraphConditionalHandle cond = 0) {
-    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
-    const Tiling tl = make_tiling(d, 8 * PhaseCheck::R);
-    PF_LAUNCH("spectral_check", s, launch_pdl(spectral_check, dim3(tiled_grid(tl)), dim3(32, 8), 0, s,
-                                              d, tl, lap_coef<double>(g), sc, part, src, x, c1, c2,
-                                              min_res, max_it, use_cond, cond));
 }
 
 // p += DP (src/solver/pressure.py:294)
@@ -1047,18 +1221,17 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
         SpectralPlan sp;
         if (spectral_setup(g, ptr, &sp) != cudaSuccess ||
             spectral_enqueue_tables(sp, s) != cudaSuccess ||
-            spectral_enqueue_solve(sp, source, c1 * c2, DP, s) != cudaSuccess)
+            spectral_enqueue_solve(sp, source, c1 * c2, DP, &sc->nonfin, s) != cudaSuccess)
             return PF_ERR_CUDA;
-        launch_spectral_check(g, sc, part, source, DP, c1, c2, min_res, max_it, s);
+        ProjectArgs A{};
+        A.sc = sc; A.part = part; A.src = source; A.c1 = c1; A.c2 = c2;
+        A.min_res = min_res; A.max_it = max_it; A.DP = DP;
+        launch_project<true, false>("spectral_check", g, A, s);
         if (cudaGetLastError() != cudaSuccess || read_scalars(sc, &hs, s)) return PF_ERR_CUDA;
         solved = hs.done != 0;
         outer = hs.max_b == 0.0 ? 0 : 1;
         total = hs.total;
         out.max_res = hs.max_res; out.iterations = total; out.outer = outer; out.status = hs.status;
-        // a non-finite right-hand side leaves DP = 0, as the iterations do
-        if (hs.status == PF_NONFINITE &&
-            cudaMemsetAsync(DP, 0, n * sizeof(double), s) != cudaSuccess)
-            return PF_ERR_CUDA;
         // the mixed forms go on from here, in FP64; PF_FP64 starts over
         warm = use64 = prec != PF_FP64;
     }
@@ -1329,35 +1502,47 @@ vel_corr_kernel(Dims d, const double* __restrict__ DP, double scale, double dxi,
 }
 
 // max|u|, max|v|, max|w|, sum(u^2+v^2+w^2), max|div u| (and, with DISS, the
-// sum of S_ij S_ij of the cell-centred strain rate): one warp per (i, j) row
-// of cells, its lanes along z (row and neighbour-row offsets computed once per
-// row).  out[3] = TKE = 0.5 <u^2 + v^2 + w^2>, out[5] = 2 nu <S_ij S_ij>.
-template <bool DISS>
-__global__ void __launch_bounds__(256)
-stats_kernel(Dims d, BicgScalars* sc, double* part, const double* __restrict__ u,
-             const double* __restrict__ v, const double* __restrict__ w,
-             double dxi, double dyi, double dzi, double nu, double* out) {
+// sum of S_ij S_ij of the cell-centred strain rate): 32 x 8 threads per tile of
+// a plane, V cells in z per thread (16-byte loads), maxima as integers.
+// out[3] = TKE = 0.5 <u^2 + v^2 + w^2>, out[5] = 2 nu <S_ij S_ij>.  INFO (step
+// graphs): out[5..9] = max_res, iterations, status of the solve in sc, += its
+// iterations, += 1; with unless_redo nothing where sc->redo says that the step
+// is not finished.  24.5 -> 18 us at 128^3 and 11.0 -> 8 at 64^3 against one
+// warp per row of cells with NaN-propagating floating-point maxima and a
+// reduction per value.
+template <int V, bool DISS, bool INFO>
+__global__ void __launch_bounds__(kBlock, DISS ? 2 : 4)
+stats_kernel(Dims d, int tz, int ty, long long ntiles, BicgScalars* sc, double* part,
+             const double* __restrict__ u, const double* __restrict__ v,
+             const double* __restrict__ w, double dxi, double dyi, double dzi, double nu,
+             int mixed, int unless_redo, double* out) {
     constexpr int NC = DISS ? 6 : 5;
-    __shared__ double sh[32];
+    __shared__ double sh[48], f[6];
+    if (INFO && unless_redo && sc->redo) return;
     double mu_ = 0, mv = 0, mw = 0, s = 0, md = 0, ss = 0;
-    const int lane = threadIdx.x & 31;
-    const int nrows = d.nx * d.ny, wpb = blockDim.x >> 5;
-    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < nrows; row += gridDim.x * wpb) {
-        const int i = row / d.ny, j = row - i * d.ny;
-        const long long base = (long long)row * d.nz;
-        const long long bx = ((long long)wrap(i + 1, d.nx) * d.ny + j) * d.nz;
-        const long long by = ((long long)i * d.ny + wrap(j + 1, d.ny)) * d.nz;
-        for (int k = lane; k < d.nz; k += 32) {
-            const long long q = base + k;
-            const double a = u[q], b = v[q], c = w[q];
-            mu_ = nanmax(mu_, fabs(a)); mv = nanmax(mv, fabs(b)); mw = nanmax(mw, fabs(c));
-            s += (a * a + b * b) + c * c;
-            double dv = (u[bx + k] - a) * dxi;
-            dv += (v[by + k] - b) * dyi;
-            dv += (w[base + wrap(k + 1, d.nz)] - c) * dzi;
-            md = nanmax(md, fabs(dv));
+    const long long plane = (long long)d.ny * d.nz;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int t1 = (int)(t / tz), i = t1 / ty;
+        const int k = ((int)(t - (long long)t1 * tz) * 32 + threadIdx.x) * V;
+        const int j = (t1 - i * ty) * 8 + threadIdx.y;
+        if (k >= d.nz || j >= d.ny) continue;
+        const long long row = i * plane + (long long)j * d.nz, q = row + k;
+        const Cells<V> a = ld_cells<V>(u + q), b = ld_cells<V>(v + q), c = ld_cells<V>(w + q);
+        const Cells<V> ax = ld_cells<V>(u + wrap(i + 1, d.nx) * plane + (long long)j * d.nz + k);
+        const Cells<V> by = ld_cells<V>(v + i * plane + (long long)wrap(j + 1, d.ny) * d.nz + k);
+        const double cz = w[row + wrap(k + V, d.nz)];
+#pragma unroll
+        for (int m = 0; m < V; ++m) {
+            mu_ = absmax(mu_, abs_bits(a.a[m]));
+            mv = absmax(mv, abs_bits(b.a[m]));
+            mw = absmax(mw, abs_bits(c.a[m]));
+            s += (a.a[m] * a.a[m] + b.a[m] * b.a[m]) + c.a[m] * c.a[m];
+            double dv = (ax.a[m] - a.a[m]) * dxi;
+            dv += (by.a[m] - b.a[m]) * dyi;
+            dv += ((m + 1 < V ? c.a[m + 1 < V ? m + 1 : m] : cz) - c.a[m]) * dzi;
+            md = absmax(md, abs_bits(dv));
             if (DISS) {
-                const Grad9 g = grad_center(d, u, v, w, i, j, k, dxi, dyi, dzi);
+                const Grad9 g = grad_center(d, u, v, w, i, j, k + m, dxi, dyi, dzi);
                 const double s12 = 0.5 * (g.uy + g.vx);
                 const double s13 = 0.5 * (g.uz + g.wx);
                 const double s23 = 0.5 * (g.vz + g.wy);
@@ -1366,21 +1551,23 @@ stats_kernel(Dims d, BicgScalars* sc, double* part, const double* __restrict__ u
             }
         }
     }
-    double r[6] = {block_max<kBlock>(mu_, sh), block_max<kBlock>(mv, sh),
-                   block_max<kBlock>(mw, sh), block_sum<kBlock>(s, sh),
-                   block_max<kBlock>(md, sh), DISS ? block_sum<kBlock>(ss, sh) : 0.0};
-    if (threadIdx.x == 0)
-        for (int c = 0; c < NC; ++c) part[c * kMaxPartials + blockIdx.x] = r[c];
-    if (arrive_last(sc)) {
-        double f[6];
-        for (int c = 0; c < NC; ++c)
-            f[c] = (c == 3 || c == 5) ? finish<false>(part + c * kMaxPartials, sh)
-                                      : finish<true>(part + c * kMaxPartials, sh);
-        if (threadIdx.x == 0) {
+    double red[NC];
+    red[0] = mu_; red[1] = mv; red[2] = mw; red[3] = s; red[4] = md;
+    if constexpr (DISS) red[5] = ss;
+    if (grid_reduce<NC, 0x17u>(red, sc, part, kPassBlocks, sh, f)) {
+        if (tid0()) {
             out[0] = f[0]; out[1] = f[1]; out[2] = f[2];
             out[3] = f[3] / double(d.n) * 0.5;
             out[4] = f[4];
             if (DISS) out[5] = 2.0 * nu * (f[5] / double(d.n));
+            if (INFO) {
+                const double it = double(mixed ? sc->total : sc->iter);
+                out[5] = sc->max_res;
+                out[6] = it;
+                out[7] = double(sc->status);
+                out[8] += it;
+                out[9] += 1.0;
+            }
             sc->counter = 0u;
         }
     }
@@ -1388,6 +1575,25 @@ stats_kernel(Dims d, BicgScalars* sc, double* part, const double* __restrict__ u
 
 size_t stats_ws_bytes(const pf_grid*) {
     return align256(sizeof(BicgScalars)) + align256(6 * kMaxPartials * sizeof(double));
+}
+
+template <bool DISS, bool INFO>
+static void launch_stats_kernel(const char* name, const pf_grid* g, const double* u,
+                                const double* v, const double* w, double nu, BicgScalars* sc,
+                                double* part, int mixed, int unless_redo, double* out,
+                                cudaStream_t s) {
+    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    const double dxi = 1.0 / g->dx, dyi = 1.0 / g->dy, dzi = 1.0 / g->dz;
+    const bool vec = g->nz % 2 == 0 && (((uintptr_t)u | (uintptr_t)v | (uintptr_t)w) & 15) == 0;
+    const int zt = vec ? 64 : 32, tz = (g->nz + zt - 1) / zt, ty = (g->ny + 7) / 8;
+    const long long nt = (long long)tz * ty * g->nx;
+    const int nb = (int)std::min<long long>(nt, kPassBlocks);
+    if (vec)
+        PF_LAUNCH(name, s, stats_kernel<2, DISS, INFO><<<nb, dim3(32, 8), 0, s>>>(
+            d, tz, ty, nt, sc, part, u, v, w, dxi, dyi, dzi, nu, mixed, unless_redo, out));
+    else
+        PF_LAUNCH(name, s, stats_kernel<1, DISS, INFO><<<nb, dim3(32, 8), 0, s>>>(
+            d, tz, ty, nt, sc, part, u, v, w, dxi, dyi, dzi, nu, mixed, unless_redo, out));
 }
 
 static cudaError_t launch_stats_impl(const pf_grid* g, const double* u, const double* v,
@@ -1398,14 +1604,17 @@ static cudaError_t launch_stats_impl(const pf_grid* g, const double* u, const do
     BicgScalars* sc = (BicgScalars*)ptr; ptr += align256(sizeof(BicgScalars));
     double* part = (double*)ptr;
     cudaMemsetAsync(sc, 0, sizeof(BicgScalars), s);
-    const double dxi = 1.0 / g->dx, dyi = 1.0 / g->dy, dzi = 1.0 / g->dz;
-    if (diss)
-        PF_LAUNCH("flow_stats", s, stats_kernel<true><<<pointwise_grid(d.n), kBlock, 0, s>>>(
-            d, sc, part, u, v, w, dxi, dyi, dzi, nu, out));
-    else
-        PF_LAUNCH("stats", s, stats_kernel<false><<<pointwise_grid(d.n), kBlock, 0, s>>>(
-            d, sc, part, u, v, w, dxi, dyi, dzi, 0.0, out));
+    if (diss) launch_stats_kernel<true, false>("flow_stats", g, u, v, w, nu, sc, part, 0, 0, out, s);
+    else launch_stats_kernel<false, false>("stats", g, u, v, w, 0.0, sc, part, 0, 0, out, s);
     return cudaGetLastError();
+}
+
+// A step graph's statistics: sc and part are the solver's (their contents but
+// the solve's result are spent by then).
+static void launch_step_stats(const pf_grid* g, const double* u, const double* v, const double* w,
+                              BicgScalars* sc, double* part, bool mixed, bool unless_redo,
+                              double* out, cudaStream_t s) {
+    launch_stats_kernel<false, true>("stats", g, u, v, w, 0.0, sc, part, mixed, unless_redo, out, s);
 }
 
 cudaError_t launch_stats(const pf_grid* g, const double* u, const double* v,
@@ -1514,19 +1723,6 @@ fold_mixed(Dims d, const BicgScalars* sc, const float* e32, const double* e64, d
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < d.n;
          q += (long long)gridDim.x * blockDim.x)
         x[q] = x[q] + s * (f64 ? e64[q] : double(e32[q]));
-}
-
-// copy the solve's result next to the monitor statistics:
-// info[0] = max_res, info[1] = iterations, info[2] = status,
-// info[3] += iterations and info[4] += 1 (running totals over launches)
-__global__ void step_info(const BicgScalars* sc, int mixed, double* info) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const double it = double(mixed ? sc->total : sc->iter);
-    info[0] = sc->max_res;
-    info[1] = it;
-    info[2] = double(sc->status);
-    info[3] += it;
-    info[4] += 1.0;
 }
 
 struct StepPlan {
@@ -1653,8 +1849,22 @@ static int plan_layout(const pf_grid* g, int prec, double min_res, const double*
     return PF_OK;
 }
 
-// After the solve (node `dep`): the result next to the statistics, p += DP, the
-// projection and the monitor statistics.
+// The monitor statistics with the solve's result next to them, after node
+// `dep`; unless_redo: nothing, where the iterations behind the direct solve run.
+static int add_stats(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g, PlanLayout& P,
+                     const double* u, const double* v, const double* w, bool mixed,
+                     bool unless_redo, double* stats, cudaStream_t cs, cudaGraphNode_t* end) {
+    int rc;
+    cudaGraph_t seg = nullptr;
+    if ((rc = capture_begin(cs, nullptr))) return rc;
+    launch_step_stats(g, u, v, w, P.sc, P.part, mixed, unless_redo, stats, cs);
+    if ((rc = capture_end(cs, &seg))) return rc;
+    rc = add_child(G, dep, seg, end);
+    cudaGraphDestroy(seg);
+    return rc;
+}
+
+// After the solve (node `dep`): p += DP, the projection, the statistics.
 static int add_step_end(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g, PlanLayout& P,
                         double* u, double* v, double* w, double* p, double* DP, double rho,
                         double dt, bool mixed, double* stats, cudaStream_t cs,
@@ -1662,14 +1872,15 @@ static int add_step_end(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g, Pl
     int rc;
     cudaGraph_t seg = nullptr;
     if ((rc = capture_begin(cs, nullptr))) return rc;
-    step_info<<<1, 32, 0, cs>>>(P.sc, mixed ? 1 : 0, stats + 5);
-    add_inplace<<<pointwise_grid(P.d.n), kBlock, 0, cs>>>(P.d.n, DP, p);
-    launch_vel_corr(g, DP, dt / rho, u, v, w, cs);
-    launch_stats(g, u, v, w, stats, P.R, cs);
+    ProjectArgs A{};
+    A.DP = DP; A.scale = dt / rho;
+    A.u = u; A.v = v; A.w = w; A.p = p;
+    launch_project<false, true>("project", g, A, cs);
     if ((rc = capture_end(cs, &seg))) return rc;
-    rc = add_child(G, dep, seg, end);
+    cudaGraphNode_t np;
+    rc = add_child(G, dep, seg, &np);
     cudaGraphDestroy(seg);
-    return rc;
+    return rc ? rc : add_stats(G, np, g, P, u, v, w, mixed, false, stats, cs, end);
 }
 
 // Adds one request's step after the predictor (node `dep`) to graph G:
@@ -1702,23 +1913,33 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
     if ((rc = capture_begin(cs, nullptr))) return rc;
     launch_div(g, u, v, w, P.div, cs);
     if (P.sp.on) {
-        // the direct solve and its check; the refinement loop below, with FP64
-        // passes only, sits in an IF node that the check opens
-        spectral_enqueue_solve(P.sp, P.div, c1 * c2, DP, cs);
-        launch_spectral_check(g, sc, part, P.div, DP, c1, c2, min_res, max_it, cs, 1, hmore);
+        // the direct solve, its check and the correction; beside the statistics
+        // an IF node that the check opens: correction taken back, the
+        // refinement loop below with FP64 passes only, and the step's end again
+        spectral_enqueue_solve(P.sp, P.div, c1 * c2, DP, &sc->nonfin, cs);
+        ProjectArgs A{};
+        A.sc = sc; A.part = part; A.src = P.div; A.c1 = c1; A.c2 = c2;
+        A.min_res = min_res; A.max_it = max_it; A.DP = DP; A.scale = dt / rho;
+        A.u = u; A.v = v; A.w = w; A.p = p;
+        A.use_cond = 1; A.cond = hmore;
+        launch_project<true, true>("project_check", g, A, cs);
         if ((rc = capture_end(cs, &seg1))) return rc;
         cudaGraphNode_t ns;
         rc = add_child(G, dep, seg1, &ns);
         cudaGraphDestroy(seg1);
         if (rc) return rc;
+        if ((rc = add_stats(G, ns, g, P, u, v, w, true, true, stats, cs, end))) return rc;
         cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
         prm.conditional.handle = hmore;
         prm.conditional.type = cudaGraphCondTypeIf;
         prm.conditional.size = 1;
-        if (cudaGraphAddNode(&nsolved, G, &ns, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
+        cudaGraphNode_t nif;
+        if (cudaGraphAddNode(&nif, G, &ns, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
         C = prm.conditional.phGraph_out[0];
         dep = nullptr;
         if ((rc = capture_begin(cs, nullptr))) return rc;
+        project_undo<<<cgrid(d), dim3(32, 8), 0, cs>>>(d, DP, dt / rho, 1.0 / g->dx, 1.0 / g->dy,
+                                                      1.0 / g->dz, u, v, w, p);
     }
     if (prec == PF_FP64) {
         const LapCoef<double> cf = lap_coef<double>(g);
@@ -1754,7 +1975,7 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
     cudaGraph_t body;
     cudaGraphConditionalHandle h;
     if ((rc = add_while(C, n1, &nw, &body, &h))) return rc;
-    if (!P.sp.on) nsolved = nw;
+    nsolved = nw;
     if (prec == PF_FP64) {
         const LapCoef<double> cf = lap_coef<double>(g);
         const Tiling ta = make_tiling(d, 8 * PhaseCA<double>::R);
@@ -1872,7 +2093,9 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
         cudaGraphDestroy(post);
         if (rc) return rc;
     }
-    return add_step_end(G, nsolved, g, P, u, v, w, p, DP, rho, dt, prec != PF_FP64, stats, cs, end);
+    cudaGraphNode_t last;
+    return add_step_end(C, nsolved, g, P, u, v, w, p, DP, rho, dt, prec != PF_FP64, stats, cs,
+                        P.sp.on ? &last : end);
 }
 
 // Captures the body of `enqueue(cs)` as a child node of G (no dependency).

@@ -50,6 +50,7 @@ struct PassArgs {
     double scale;       // c / (nx ny nz)
     const double *lamy, *lamz;
     int nz;
+    int* nonfin;        // first z pass: set where the input is not finite
 };
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -261,15 +262,20 @@ spectral_pass(PassArgs a) {
     if (KIND == kPassZ) {
         const int lane = tid & 31, nw = nt >> 5;
         const long long r0 = (long long)blockIdx.x * (2 * L);
+        double big = 0.0;
         for (int q = tid >> 5; q < L; q += nw) {
             const long long ra = r0 + 2 * q;
             if (ra >= a.nlines) break;
             const bool two = ra + 1 < a.nlines;
             const double* pa = a.src + ra * n;
 #pragma unroll 4
-            for (int e = lane; e < n; e += 32)
-                sm[slot<L>(e, q)] = make_double2(pa[e], two ? pa[n + e] : 0.0);
+            for (int e = lane; e < n; e += 32) {
+                const double2 x = make_double2(pa[e], two ? pa[n + e] : 0.0);
+                sm[slot<L>(e, q)] = x;
+                big = absmax(big, absmax(abs_bits(x.x), abs_bits(x.y)));
+            }
         }
+        if (a.nonfin && !(big < __longlong_as_double(0x7ff0000000000000LL))) *a.nonfin = 1;
     } else {
         long long plane = 0;
         if (KIND == kPassY) {
@@ -523,13 +529,14 @@ cudaError_t spectral_enqueue_tables(const SpectralPlan& P, cudaStream_t s) {
 }
 
 cudaError_t spectral_enqueue_solve(const SpectralPlan& P, const double* src, double c, double* DP,
-                                   cudaStream_t s) {
+                                   int* nonfin, cudaStream_t s) {
     const Dims& d = P.d;
     const bool al = ((uintptr_t)DP & 15) == 0;
     auto pairs = [](long long lines) { return (lines + 1) / 2; };
     PassArgs z{};
     z.ax = P.ax[2];
     z.src = src; z.dst = DP;
+    z.nonfin = nonfin;
     z.nlines = (long long)d.nx * d.ny;
     z.stride = 1;
     const long long bz = (pairs(z.nlines) + z.ax.lines - 1) / z.ax.lines;
@@ -556,6 +563,7 @@ cudaError_t spectral_enqueue_solve(const SpectralPlan& P, const double* src, dou
     launch_pass<kPassX>("spectral_x", x, bx, s);
     launch_pass<kPassY>("spectral_y", y, by, s);
     z.src = DP;
+    z.nonfin = nullptr;
     launch_pass<kPassZ>("spectral_z", z, bz, s);
     return cudaGetLastError();
 }

@@ -43,8 +43,9 @@ size_t spectral_table_bytes(const pf_grid* g);
 cudaError_t spectral_setup(const pf_grid* g, void* tables, SpectralPlan* P);
 // Fills the tables (once per plan, or before a solve).
 cudaError_t spectral_enqueue_tables(const SpectralPlan& P, cudaStream_t s);
-// DP = the zero-mean solution of A DP = c src (c = -vol rho / dt).
+// DP = the zero-mean solution of A DP = c src (c = -vol rho / dt); *nonfin
+// becomes 1 where src holds a NaN or Inf (and is left alone otherwise).
 cudaError_t spectral_enqueue_solve(const SpectralPlan& P, const double* src, double c, double* DP,
-                                   cudaStream_t s);
+                                   int* nonfin, cudaStream_t s);
 
 }  // namespace pf

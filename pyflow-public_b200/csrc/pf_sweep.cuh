@@ -22,6 +22,8 @@ struct BicgScalars {
     unsigned int counter;
     int use64;          // mixed graph mode: the next refinement pass runs in FP64
     double prev_ratio;  // mixed graph mode: true residual ratio after the previous pass
+    int nonfin;         // direct solve: a NaN or Inf in the right-hand side
+    int redo;           // direct solve, graph mode: the iterations behind it run
 };
 
 template <typename T>

@@ -100,3 +100,42 @@ def test_unaligned_fields():
     want = _exact(a, sp)
     assert info.status == 0
     assert np.linalg.norm(DP.cpu().numpy() - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("shape", [(40, 36, 24), (21, 20, 33)])
+def test_plan_takes_the_correction_back(shape):
+    """A box flattened in z whose flow does not vary in z: the rounding of
+    A x, times the square of the aspect ratio, is above the tolerance, so the
+    step graph's check fails after the correction, which is taken back before
+    the FP64 passes run and is applied again.  The limit ends them; velocity
+    and pressure are those of the host-driven step, which corrects once."""
+    import pyflow_b200.ops as ops
+    from pyflow_b200.plan import StepPlan
+    sp = (0.2, 0.25, 2e-6)
+    rng = np.random.default_rng(5)
+    k = [2 * np.pi * np.arange(n) / n for n in shape[:2]]
+    f0 = [np.broadcast_to((np.sin(k[0] + a)[:, None] * np.cos(k[1] + b)[None, :])[..., None], shape)
+          for a, b in rng.uniform(0, 6, (3, 2))]
+    f0 = [torch.tensor(np.ascontiguousarray(x), device="cuda") for x in f0]
+    out = []
+    for plan in (True, False):
+        f = [t.clone() for t in f0] + [torch.zeros_like(f0[0]), torch.zeros_like(f0[0])]
+        if plan:
+            pl = StepPlan(*f, sp, 0.0, 1.0, 1e-7, min_res=1e-10, max_it=12, prec="mixed")
+            pl.launch(1)
+            torch.cuda.synchronize()
+            st = pl.stats()
+            pl.close()
+            status, res = int(st["status"]), st["max_res"]
+            np.testing.assert_allclose(
+                [st[n] for n in ("max_u", "max_v", "max_w", "tke", "max_div")],
+                ops.stats(*f[:3], sp).cpu().numpy(), rtol=1e-14)
+        else:
+            info = ops.forward_step(*f, sp, 0.0, 1.0, 1e-7, min_res=1e-10, max_it=12, prec="mixed")
+            status, res = info.status, info.max_res
+        out.append((f, status, res))
+    (a, sa, ra), (b, sb, rb) = out
+    assert sa != 0 and sb != 0 and ra > 1e-10 and rb > 1e-10
+    for x, y in zip(a[:4], b[:4]):
+        assert torch.isfinite(x).all()
+        assert float((x - y).abs().max()) <= 1e-6 * float(y.abs().max())
