@@ -245,6 +245,28 @@ int pf_rhs_adjoint(const pf_grid* g, const double* u, const double* v,
  * dL/d(FXX, FYY, FZZ, FXY, FXZ, FYZ) for the RHS adjoint mu.  FP64. */
 int pf_sfs_adjoint(const pf_grid* g, const double* mu_u, const double* mu_v,
                    const double* mu_w, double weight, double* out, void* stream);
+/* Vector-Jacobian product of pf_predictor_step (FP64, constant viscosity, sfs
+ * stresses or NULL) at the step input u, v, w: out = dL/d(u, v, w) for the
+ * predictor's adjoint input lam, stage states recomputed; out_sfs (six fields,
+ * or NULL) = dL/dsfs.  lam and out must not overlap.  Asynchronous; ws of
+ * pf_predictor_vjp_workspace_bytes. */
+size_t pf_predictor_vjp_workspace_bytes(const pf_grid* g);
+int pf_predictor_vjp(const pf_grid* g, int rk4, const double* u, const double* v,
+                     const double* w, const double* lam_u, const double* lam_v,
+                     const double* lam_w, double mu, double rho, double dt,
+                     const double* sfs, double* out_u, double* out_v,
+                     double* out_w, double* out_sfs, void* ws, size_t ws_bytes,
+                     void* stream);
+/* The projection of Domain.TargetDataVelCorr (src/data/domain.py:445-468) in
+ * one call, FP64, solved directly (PF_DIRECT_SOLVE): u, v, w -= dt/rho grad DP,
+ * p += DP.  A field whose divergence is round-off of it (max|div| <= 1e-9
+ * max|velocity| / smallest spacing) is left alone, with DP = 0 and *skipped
+ * = 1.  Synchronous; ws of pf_workspace_bytes(g, PF_FP64). */
+int pf_project(const pf_grid* g, double* u, double* v, double* w, double* DP,
+               double* p, double rho, double dt, double min_res, int max_it,
+               void* ws, size_t ws_bytes, void* stream, pf_solve_info* info,
+               int* skipped);
+
 
 /* No counterpart in the reference: the pf_bicgstab_solve solve (FP64) for
  * callers that cannot allocate device memory or pass a workspace (for example

@@ -38,6 +38,15 @@ _lib.pf_rhs_adjoint.argtypes = [_G, _P, _P, _P, _P, _P, _P, _D, _D, _P, _P, _P, 
 _lib.pf_rhs_adjoint.restype = ctypes.c_int
 _lib.pf_sfs_adjoint.argtypes = [_G, _P, _P, _P, _D, _P, _P]
 _lib.pf_sfs_adjoint.restype = ctypes.c_int
+_I, _S = ctypes.c_int, ctypes.c_size_t
+_lib.pf_predictor_vjp_workspace_bytes.argtypes = [_G]
+_lib.pf_predictor_vjp_workspace_bytes.restype = _S
+_lib.pf_predictor_vjp.argtypes = [_G, _I, _P, _P, _P, _P, _P, _P, _D, _D, _D, _P, _P, _P, _P, _P,
+                                  _P, _S, _P]
+_lib.pf_predictor_vjp.restype = _I
+_lib.pf_project.argtypes = [_G, _P, _P, _P, _P, _P, _D, _D, _D, _I, _P, _S, _P,
+                            ctypes.POINTER(L.SolveInfo), ctypes.POINTER(_I)]
+_lib.pf_project.restype = _I
 
 
 def rhs_adjoint(state, lam, spacing, mu, rho):
@@ -67,21 +76,28 @@ def project(vel, spacing, rho, dt, tol=1e-12, max_it=20000, p=None, DP=None):
     reference's solve also adds DP to the pressure it is given (the
     simulation's p): pass ``p`` to get that; ``DP`` receives the solution."""
     u, v, w = vel
-    DP = torch.zeros_like(u) if DP is None else DP.zero_()
+    for t, nm in ((u, "u"), (v, "v"), (w, "w")):
+        ops._check(t, u.shape, torch.float64, nm)
+    DP = torch.empty_like(u) if DP is None else DP
     p = torch.zeros_like(u) if p is None else p
+    for t, nm in ((DP, "DP"), (p, "p")):
+        ops._check(t, u.shape, torch.float64, nm)
     # a field that is already divergence free to the solver's precision (the
     # adjoint of a loss between two projected fields: its divergence is
     # round-off of the field) needs no correction: a solve of a round-off
     # right-hand side (whose mean is not zero) only iterates on noise,
     # stagnates at the relative tolerance and can end non-finite
-    mu, mv, mw, _, mdiv = ops.stats(u, v, w, spacing).tolist()
-    if mdiv <= 1e-9 * max(mu, mv, mw) / min(spacing):
+    g = ops.grid(u.shape, spacing)
+    ws = ops.workspace(g, L.PF_FP64, u.device)
+    info, skipped = L.SolveInfo(), _I(0)
+    L.check("pf_project", _lib.pf_project(
+        ctypes.byref(g), ops._p(u), ops._p(v), ops._p(w), ops._p(DP), ops._p(p), float(rho),
+        float(dt), float(tol), int(max_it), ops._p(ws), ws.numel(), ops._stream(u),
+        ctypes.byref(info), ctypes.byref(skipped)))
+    if skipped.value:
         return None
-    src = ops.div_vel(u, v, w, spacing)
-    info = ops.bicgstab_solve(src, DP, p, spacing, rho, dt, tol, max_it, direct=True)
     if info.status == L.PF_NONFINITE:
         raise RuntimeError("projection solve: non-finite residual")
-    ops.vel_corr(DP, dt / rho, u, v, w, spacing)
     return info
 
 
@@ -153,12 +169,35 @@ def _source_vjp(source, stage, kbar):
     return tuple(t.grad if t.grad is not None else torch.zeros_like(t) for t in x)
 
 
+def predictor_vjp(state, lam, spacing, mu, rho, dt, sfs=None, rk4=True):
+    """The predictor's vector-Jacobian product at the step input ``state`` for
+    the (projected) adjoint field ``lam``, in one library call
+    (pf_predictor_vjp): dL/du_n and, with ``sfs``, dL/dF."""
+    for t in (*state, *lam):
+        ops._check(t, state[0].shape, torch.float64, "state and adjoint")
+    u = state[0]
+    if sfs is not None:
+        ops._check(sfs, (6,) + tuple(u.shape), torch.float64, "sfs")
+    g = ops.grid(u.shape, spacing)
+    need = _lib.pf_predictor_vjp_workspace_bytes(ctypes.byref(g))
+    ws = torch.empty(need, dtype=torch.uint8, device=u.device)
+    out = tuple(torch.empty_like(u) for _ in range(3))
+    lamF = torch.empty_like(sfs) if sfs is not None else None
+    L.check("pf_predictor_vjp", _lib.pf_predictor_vjp(
+        ctypes.byref(g), 1 if rk4 else 0, *(ops._p(t) for t in (*state, *lam)), float(mu),
+        float(rho), float(dt), ops._p(sfs), *(ops._p(t) for t in out), ops._p(lamF), ops._p(ws),
+        need, ops._stream(u)))
+    return out, lamF
+
+
 def step_vjp(state, lam_out, spacing, mu, rho, dt, sfs=None, rk4=True,
              tol=1e-12, max_it=20000, source=None):
     """dL/du_n given dL/du_{n+1} (and dL/dF of the SFS stresses if sfs; a
     'source' closure's parameter gradients accumulate in its parameters)."""
     lam = tuple(t.clone() for t in lam_out)
     project(lam, spacing, rho, dt, tol, max_it)            # lam* = P lam
+    if source is None:
+        return predictor_vjp(state, lam, spacing, mu, rho, dt, sfs, rk4)
     stages = stage_states(state, spacing, mu, rho, dt, sfs, rk4, source)
     lamF = torch.zeros((6,) + tuple(state[0].shape), dtype=torch.float64,
                        device=state[0].device) if sfs is not None else None

@@ -32,18 +32,17 @@ struct AdjArgs {
     double dxi, dyi, dzi;
     double a;   // 2 mu / rho   (diagonal viscous flux factor)
     double e;   // mu_edge / rho (off-diagonal viscous flux factor)
+    double scale;  // of the adjoint input
 };
 
-__global__ void __launch_bounds__(256)
-rhs_adjoint_kernel(Dims d, AdjArgs A, double* __restrict__ ou,
-                   double* __restrict__ ov, double* __restrict__ ow) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z;
-    if (k >= d.nz || j >= d.ny) return;
+// J(state)^T lambda of one cell; lambda = A.scale * (mu, mv, mw), the product
+// rounded first (A.scale 1: lambda itself).
+__device__ __forceinline__ void rhs_adjoint_cell(const Dims& d, const AdjArgs& A, int i, int j,
+                                                 int k, double& ru, double& rv, double& rw) {
     const double dxi = A.dxi, dyi = A.dyi, dzi = A.dzi;
     auto at = [&](const double* f, int di, int dj, int dk) -> double {
-        return __ldg(f + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
+        const double x = __ldg(f + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
+        return f == A.mu || f == A.mv || f == A.mw ? A.scale * x : x;
     };
     // ---- convective flux adjoints (at flux position p = c + (di,dj,dk))
     auto lamCxx = [&](int di, int dj, int dk) { return dxi * (at(A.mu, di + 1, dj, dk) - at(A.mu, di, dj, dk)); };
@@ -125,10 +124,20 @@ rhs_adjoint_kernel(Dims d, AdjArgs A, double* __restrict__ ou,
     av += dxi * (txy(-1, 0, 0) - txy(0, 0, 0)) + dzi * (tyz(0, 0, -1) - tyz(0, 0, 0));
     aw += dxi * (txz(-1, 0, 0) - txz(0, 0, 0)) + dyi * (tyz(0, -1, 0) - tyz(0, 0, 0));
 
+    ru = au;
+    rv = av;
+    rw = aw;
+}
+
+__global__ void __launch_bounds__(256)
+rhs_adjoint_kernel(Dims d, AdjArgs A, double* __restrict__ ou,
+                   double* __restrict__ ov, double* __restrict__ ow) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= d.nz || j >= d.ny) return;
     const long long q = idx(d, i, j, k);
-    ou[q] = au;
-    ov[q] = av;
-    ow[q] = aw;
+    rhs_adjoint_cell(d, A, i, j, k, ou[q], ov[q], ow[q]);
 }
 
 // Adjoint of the 'tensor' SFS stresses: the stresses are added to the viscous
@@ -137,16 +146,12 @@ rhs_adjoint_kernel(Dims d, AdjArgs A, double* __restrict__ ou,
 // centres one cell below (interp_sc_xy, metric_staggered.py:127-144).
 // out[0..5] += adjoint of FXX, FYY, FZZ, FXY, FXZ, FYZ for adjoint mu (scaled
 // by `weight`, accumulated so that RK4 stages can be summed).
-__global__ void __launch_bounds__(256)
-sfs_adjoint_kernel(Dims d, const double* __restrict__ mu, const double* __restrict__ mv,
-                   const double* __restrict__ mw, double dxi, double dyi, double dzi,
-                   double weight, double* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z;
-    if (k >= d.nz || j >= d.ny) return;
-    auto at = [&](const double* f, int di, int dj, int dk) -> double {
-        return __ldg(f + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
+__device__ __forceinline__ void sfs_adjoint_cell(const Dims& d, const double* mu, const double* mv,
+                                                 const double* mw, double scale, double dxi,
+                                                 double dyi, double dzi, int i, int j, int k,
+                                                 double (&f)[6]) {
+    auto at = [&](const double* a, int di, int dj, int dk) -> double {
+        return scale * __ldg(a + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
     };
     // flux adjoints at edge positions p
     auto lxy = [&](int di, int dj) {
@@ -158,20 +163,65 @@ sfs_adjoint_kernel(Dims d, const double* __restrict__ mu, const double* __restri
     auto lyz = [&](int dj, int dk) {
         return dzi * (at(mv, 0, dj, dk) - at(mv, 0, dj, dk + 1)) + dyi * (at(mw, 0, dj, dk) - at(mw, 0, dj + 1, dk));
     };
-    const long long q = idx(d, i, j, k), n = d.n;
-    const double fxx = dxi * (at(mu, 0, 0, 0) - at(mu, 1, 0, 0));
-    const double fyy = dyi * (at(mv, 0, 0, 0) - at(mv, 0, 1, 0));
-    const double fzz = dzi * (at(mw, 0, 0, 0) - at(mw, 0, 0, 1));
+    f[0] = dxi * (at(mu, 0, 0, 0) - at(mu, 1, 0, 0));
+    f[1] = dyi * (at(mv, 0, 0, 0) - at(mv, 0, 1, 0));
+    f[2] = dzi * (at(mw, 0, 0, 0) - at(mw, 0, 0, 1));
     // S(p) = 0.25 (F(p) + F(p-x) + F(p-y) + F(p-x-y)): F(c) feeds p = c, c+x, c+y, c+x+y
-    const double fxy = 0.25 * (lxy(0, 0) + lxy(1, 0) + lxy(0, 1) + lxy(1, 1));
-    const double fxz = 0.25 * (lxz(0, 0) + lxz(1, 0) + lxz(0, 1) + lxz(1, 1));
-    const double fyz = 0.25 * (lyz(0, 0) + lyz(1, 0) + lyz(0, 1) + lyz(1, 1));
-    out[q] += weight * fxx;
-    out[n + q] += weight * fyy;
-    out[2 * n + q] += weight * fzz;
-    out[3 * n + q] += weight * fxy;
-    out[4 * n + q] += weight * fxz;
-    out[5 * n + q] += weight * fyz;
+    f[3] = 0.25 * (lxy(0, 0) + lxy(1, 0) + lxy(0, 1) + lxy(1, 1));
+    f[4] = 0.25 * (lxz(0, 0) + lxz(1, 0) + lxz(0, 1) + lxz(1, 1));
+    f[5] = 0.25 * (lyz(0, 0) + lyz(1, 0) + lyz(0, 1) + lyz(1, 1));
+}
+
+__global__ void __launch_bounds__(256)
+sfs_adjoint_kernel(Dims d, const double* __restrict__ mu, const double* __restrict__ mv,
+                   const double* __restrict__ mw, double dxi, double dyi, double dzi,
+                   double weight, double* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= d.nz || j >= d.ny) return;
+    double f[6];
+    sfs_adjoint_cell(d, mu, mv, mw, 1.0, dxi, dyi, dzi, i, j, k, f);
+    const long long q = idx(d, i, j, k);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) out[c * d.n + q] += weight * f[c];
+}
+
+// One stage of the reversed predictor: m = J(stage state)^T kbar with kbar =
+// A.scale * (A.mu, A.mv, A.mw); total = base + m; the next (earlier) stage's
+// kbar' = wnext lam + h m; with SFS stresses their adjoint F (+)= of kbar.  As
+// separate torch operations the four stages of a step took 70 launches and,
+// at 64^3, 0.3 ms of host time against 0.15 ms of these kernels.
+struct VjpStage {
+    const double* lam[3];   // the projected adjoint field
+    const double* base[3];  // total so far (lam at the last stage)
+    double* total[3];
+    double* next[3];        // null: no earlier stage
+    double wnext, h;
+    double* F;              // null: no SFS stresses
+    int add;                // F holds the later stages' sum
+};
+
+__global__ void __launch_bounds__(256, 2)
+vjp_stage_kernel(Dims d, AdjArgs A, VjpStage S) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z;
+    if (k >= d.nz || j >= d.ny) return;
+    const long long q = idx(d, i, j, k);
+    double m[3];
+    rhs_adjoint_cell(d, A, i, j, k, m[0], m[1], m[2]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if (S.next[c]) S.next[c][q] = S.wnext * S.lam[c][q] + S.h * m[c];
+        S.total[c][q] = S.base[c][q] + m[c];
+    }
+    if (S.F) {
+        double f[6];
+        sfs_adjoint_cell(d, A.mu, A.mv, A.mw, A.scale, A.dxi, A.dyi, A.dzi, i, j, k, f);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S.F[c * d.n + q] = S.add ? S.F[c * d.n + q] + f[c] : f[c];
+    }
 }
 
 }  // namespace pf
@@ -187,7 +237,7 @@ extern "C" int pf_rhs_adjoint(const pf_grid* g, const double* u, const double* v
         return PF_ERR_BAD_ARG;
     pf::Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
     pf::AdjArgs A{u, v, w, mu_u, mu_v, mu_w, 1.0 / g->dx, 1.0 / g->dy, 1.0 / g->dz,
-                  (2.0 * mu) / rho, (0.25 * (((mu + mu) + mu) + mu)) / rho};
+                  (2.0 * mu) / rho, (0.25 * (((mu + mu) + mu) + mu)) / rho, 1.0};
     cudaStream_t s = (cudaStream_t)stream;
     dim3 blk(32, 8), grd((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx);
     PF_LAUNCH("rhs_adjoint", s, pf::rhs_adjoint_kernel<<<grd, blk, 0, s>>>(d, A, out_u, out_v, out_w));
@@ -205,5 +255,59 @@ extern "C" int pf_sfs_adjoint(const pf_grid* g, const double* mu_u,
     dim3 blk(32, 8), grd((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx);
     PF_LAUNCH("sfs_adjoint", s, pf::sfs_adjoint_kernel<<<grd, blk, 0, s>>>(
         d, mu_u, mu_v, mu_w, 1.0 / g->dx, 1.0 / g->dy, 1.0 / g->dz, weight, out));
+    return cudaGetLastError() == cudaSuccess ? PF_OK : PF_ERR_CUDA;
+}
+
+extern "C" size_t pf_predictor_vjp_workspace_bytes(const pf_grid* g) {
+    if (!g || g->nx < 2 || g->ny < 2 || g->nz < 2) return 0;
+    // three stage states, two sets of stage adjoints
+    return (size_t)15 * g->nx * g->ny * g->nz * sizeof(double);
+}
+
+extern "C" int pf_predictor_vjp(const pf_grid* g, int rk4, const double* u, const double* v,
+                                const double* w, const double* lam_u, const double* lam_v,
+                                const double* lam_w, double mu, double rho, double dt,
+                                const double* sfs, double* out_u, double* out_v, double* out_w,
+                                double* out_sfs, void* ws, size_t ws_bytes, void* stream) {
+    if (!g || g->nx < 2 || g->ny < 2 || g->nz < 2 || !(g->dx > 0) || !(g->dy > 0) ||
+        !(g->dz > 0) || !u || !v || !w || !lam_u || !lam_v || !lam_w || !out_u || !out_v ||
+        !out_w || !(rho != 0.0) || !ws || ((uintptr_t)ws & 7) ||
+        ws_bytes < pf_predictor_vjp_workspace_bytes(g) || (out_sfs && !sfs))
+        return PF_ERR_BAD_ARG;
+    using namespace pf;
+    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    const long long n = d.n;
+    cudaStream_t s = (cudaStream_t)stream;
+    double* st = (double*)ws;
+    double* kb[2] = {st + 9 * n, st + 12 * n};
+    const int stages = rk4 ? 4 : 1;
+    if (rk4 && launch_stage_states(g, u, v, w, mu, rho, sfs, dt, st, s) != cudaSuccess)
+        return PF_ERR_CUDA;
+    const double* lam[3] = {lam_u, lam_v, lam_w};
+    double* out[3] = {out_u, out_v, out_w};
+    const double wts[4] = {dt / 6.0, dt / 3.0, dt / 3.0, dt / 6.0};
+    dim3 blk(32, 8), grd((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx);
+    for (int q = stages - 1; q >= 0; --q) {
+        const double* x = q ? st + 3 * n * (q - 1) : nullptr;
+        const bool first = q == stages - 1;
+        const double* kin = kb[q & 1];
+        AdjArgs A{x ? x : u, x ? x + n : v, x ? x + 2 * n : w,
+                  first ? lam_u : kin, first ? lam_v : kin + n, first ? lam_w : kin + 2 * n,
+                  1.0 / g->dx, 1.0 / g->dy, 1.0 / g->dz, (2.0 * mu) / rho,
+                  (0.25 * (((mu + mu) + mu) + mu)) / rho,
+                  first ? (rk4 ? wts[3] : dt) : 1.0};
+        VjpStage S;
+        for (int c = 0; c < 3; ++c) {
+            S.lam[c] = lam[c];
+            S.base[c] = first ? lam[c] : out[c];
+            S.total[c] = out[c];
+            S.next[c] = q ? kb[(q - 1) & 1] + c * n : nullptr;
+        }
+        S.wnext = q ? wts[q - 1] : 0.0;
+        S.h = 0.5 * dt;
+        S.F = out_sfs;
+        S.add = first ? 0 : 1;
+        PF_LAUNCH("vjp_stage", s, vjp_stage_kernel<<<grd, blk, 0, s>>>(d, A, S));
+    }
     return cudaGetLastError() == cudaSuccess ? PF_OK : PF_ERR_CUDA;
 }

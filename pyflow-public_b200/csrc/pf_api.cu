@@ -151,6 +151,16 @@ int pf_forward_step(const pf_grid* g, int prec, int rk4, int solver,
     return PF_OK;
 }
 
+int pf_project(const pf_grid* g, double* u, double* v, double* w, double* DP, double* p,
+               double rho, double dt, double min_res, int max_it, void* ws, size_t ws_bytes,
+               void* stream, pf_solve_info* info, int* skipped) {
+    if (!grid_ok(g) || !u || !v || !w || !DP || !p || !info || !skipped || !(rho != 0.0) ||
+        !(dt != 0.0))
+        return PF_ERR_BAD_ARG;
+    if (!ws || ws_bytes < pf_workspace_bytes(g, PF_FP64)) return PF_ERR_BAD_ARG;
+    return project_solve(g, u, v, w, DP, p, rho, dt, min_res, max_it, ws, S(stream), info, skipped);
+}
+
 int pf_stats(const pf_grid* g, const double* u, const double* v,
              const double* w, double* out_dev, void* ws, size_t ws_bytes,
              void* stream) {

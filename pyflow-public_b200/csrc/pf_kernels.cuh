@@ -27,6 +27,10 @@ cudaError_t launch_predictor(const pf_grid* g, int prec, int rk4, double* u,
                              double mu, double rho, const void* sfs,
                              double dt, void* ws, cudaStream_t s);
 
+cudaError_t launch_stage_states(const pf_grid* g, const double* u, const double* v,
+                                const double* w, double mu, double rho, const double* sfs,
+                                double dt, double* st, cudaStream_t s);
+
 // One request of a grouped predictor: its grid, state, constants and the
 // stage-buffer region of its workspace (predictor_ws_bytes of it).
 struct GroupMember {
@@ -55,6 +59,9 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
                    double min_res, int max_it, const double* source,
                    double* DP, double* p, void* ws, cudaStream_t s,
                    pf_solve_info* info);
+int project_solve(const pf_grid* g, double* u, double* v, double* w, double* DP, double* p,
+                  double rho, double dt, double min_res, int max_it, void* ws, cudaStream_t s,
+                  pf_solve_info* info, int* skipped);
 int jacobi_solve(const pf_grid* g, double rho, double dt, int n_it,
                  const double* source, double* pold, double* p, void* ws,
                  cudaStream_t s, double* max_res);

@@ -1652,6 +1652,64 @@ cudaError_t launch_vel_corr(const pf_grid* g, const double* DP, double scale,
 }
 
 
+// Projection of a velocity field (pf_project): statistics, divergence, direct
+// solve and its check go out together and the host waits once for all of
+// their results; then the correction.
+int project_solve(const pf_grid* g, double* u, double* v, double* w, double* DP, double* p,
+                  double rho, double dt, double min_res, int max_it, void* ws, cudaStream_t s,
+                  pf_solve_info* info, int* skipped) {
+    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    const size_t n = (size_t)d.n;
+    double* div = (double*)ws;
+    char* ptr = (char*)ws + align256(n * sizeof(double));
+    char* rest = ptr;
+    BicgScalars* sc = (BicgScalars*)ptr; ptr += align256(sizeof(BicgScalars));
+    double* part = (double*)ptr; ptr += align256(kNumPartials * kMaxPartials * sizeof(double));
+    const double vol = (g->dx * g->dy) * g->dz;
+    const double hmin = std::min(g->dx, std::min(g->dy, g->dz));
+    struct { BicgScalars sc; char pad[192 - sizeof(BicgScalars)]; double st[5]; } h;
+    double* st = (double*)((char*)sc + 192);  // behind the scalars, in their 256 bytes
+    static_assert(sizeof(BicgScalars) <= 192, "scalar block");
+    const bool direct = spectral_applies(g, min_res, DP, ptr);
+    if (cudaMemsetAsync(sc, 0, sizeof(BicgScalars), s) != cudaSuccess) return PF_ERR_CUDA;
+    launch_stats_kernel<false, false>("stats", g, u, v, w, 0.0, sc, part, 0, 0, st, s);
+    launch_div(g, u, v, w, div, s);
+    if (direct) {
+        SpectralPlan sp;
+        if (spectral_setup(g, ptr, &sp) != cudaSuccess ||
+            spectral_enqueue_tables(sp, s) != cudaSuccess ||
+            spectral_enqueue_solve(sp, div, rho / dt * (-1.0 * vol), DP, &sc->nonfin, s) != cudaSuccess)
+            return PF_ERR_CUDA;
+        ProjectArgs A{};
+        A.sc = sc; A.part = part; A.src = div; A.c1 = rho / dt; A.c2 = -1.0 * vol;
+        A.min_res = min_res; A.max_it = std::max(max_it, 1); A.DP = DP;
+        launch_project<true, false>("spectral_check", g, A, s);
+    }
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return PF_ERR_CUDA;
+    const double vmax = std::max(h.st[0], std::max(h.st[1], h.st[2]));
+    *skipped = h.st[4] <= 1e-9 * vmax / hmin;
+    *info = pf_solve_info{0.0, 0, 1, PF_OK};
+    if (*skipped)
+        return cudaMemsetAsync(DP, 0, n * sizeof(double), s) == cudaSuccess ? PF_OK : PF_ERR_CUDA;
+    if (direct && h.sc.done && h.sc.status == PF_OK) {
+        info->max_res = h.sc.max_res;
+        info->iterations = h.sc.total;
+        ProjectArgs A{};
+        A.DP = DP; A.scale = dt / rho;
+        A.u = u; A.v = v; A.w = w; A.p = p;
+        launch_project<false, true>("project", g, A, s);
+        return cudaGetLastError() == cudaSuccess ? PF_OK : PF_ERR_CUDA;
+    }
+    // what the direct solve does not settle: the whole solve with its iterations
+    const int rc = bicgstab_solve(g, PF_FP64, rho, dt, min_res, max_it, div, DP, p, rest, s, info);
+    if (rc) return rc;
+    if (info->status == PF_NONFINITE) return PF_OK;
+    return launch_vel_corr(g, DP, dt / rho, u, v, w, s) == cudaSuccess ? PF_OK : PF_ERR_CUDA;
+}
+
 // ============================================================================
 // Whole time step as one CUDA graph.
 //

@@ -74,7 +74,8 @@ __device__ inline void rhs_cell(const Dims& d, const RhsArgs<T, TI>& a, int i, i
                 ru, rv, rw);
 }
 
-enum StageMode { kModeRhs = 0, kModeFirst = 1, kModeMid = 2, kModeLast = 3, kModeK = 4 };
+enum StageMode { kModeRhs = 0, kModeFirst = 1, kModeMid = 2, kModeLast = 3, kModeK = 4,
+                 kModeState = 5 };  // the next stage state alone (no k-sum)
 
 // Stage arithmetic of one cell (the epilogue of every stage kernel).
 template <typename T, typename TS, typename TA, int MODE>
@@ -84,14 +85,14 @@ __device__ __forceinline__ void stage_store(long long q, T ku, T kv, T kw, doubl
                                             double hdt, double c6) {
     if (MODE == kModeRhs) {
         ru[q] = ku; rv[q] = kv; rw[q] = kw;
-    } else if (MODE == kModeFirst || MODE == kModeMid) {
+    } else if (MODE == kModeFirst || MODE == kModeMid || MODE == kModeState) {
         // ZAXPY(h, k, u) = h*k + u (src/data/state.py:157-165)
         su[q] = TS(hdt * double(ku) + u[q]);
         sv[q] = TS(hdt * double(kv) + v[q]);
         sw[q] = TS(hdt * double(kw) + w[q]);
         if (MODE == kModeFirst) {
             au[q] = TA(ku); av[q] = TA(kv); aw[q] = TA(kw);
-        } else {
+        } else if (MODE == kModeMid) {
             au[q] = TA(T(au[q]) + T(2.0) * ku);
             av[q] = TA(T(av[q]) + T(2.0) * kv);
             aw[q] = TA(T(aw[q]) + T(2.0) * kw);
@@ -163,7 +164,8 @@ struct RhsSmem {
     // FP64 input planes of an FP32 stage (the state u of the first stage or
     // of Euler's k) are staged as FP64 and converted to T once per position
     static constexpr bool kConv = sizeof(TI) > sizeof(T);
-    static constexpr bool kU = MODE == kModeFirst || MODE == kModeMid || MODE == kModeLast;
+    static constexpr bool kU = MODE == kModeFirst || MODE == kModeMid || MODE == kModeLast ||
+                               MODE == kModeState;
     static constexpr bool kA = MODE == kModeMid || MODE == kModeLast;
     static constexpr size_t kEu = (kU && !kConv) ? 2 * 3 * kRhsCells * sizeof(double) : 0;  // [2][3][cells]
     static constexpr size_t kStg = kConv ? 4 * 3 * kRhsPos * sizeof(TI) : 0;             // [4][3][pos]
@@ -474,11 +476,11 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
                     const T kf = k3[r][f];
-                    if (MODE == kModeFirst || MODE == kModeMid) {
+                    if (MODE == kModeFirst || MODE == kModeMid || MODE == kModeState) {
                         // ZAXPY(h, k, u) = h*k + u (src/data/state.py:157-165)
                         S[f][q] = TS(hdt * double(kf) + eu[(buf * 3 + f) * kRhsCells + cc]);
                         if (MODE == kModeFirst) A[f][q] = TA(kf);
-                        else A[f][q] = TA(T(ea[(buf * 3 + f) * kRhsCells + cc]) + T(2.0) * kf);
+                        else if (MODE == kModeMid) A[f][q] = TA(T(ea[(buf * 3 + f) * kRhsCells + cc]) + T(2.0) * kf);
                     } else if (MODE == kModeLast) {
                         U[f][q] = eu[(buf * 3 + f) * kRhsCells + cc] +
                                   c6 * (double(T(ea[(buf * 3 + f) * kRhsCells + cc]) + kf));
@@ -714,6 +716,25 @@ static cudaError_t predictor_impl(const pf_grid* g, int rk4, double* u,
                                acc, hdt, c6, s);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
+}
+
+// The RK4 stage states u2, u3, u4 of the FP64 predictor (u_s = h k_{s-1} + u,
+// h = dt/2), three fields each at st + 3 n (s - 2).
+cudaError_t launch_stage_states(const pf_grid* g, const double* u, const double* v,
+                                const double* w, double mu, double rho, const double* sfs,
+                                double dt, double* st, cudaStream_t s) {
+    const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
+    const double *a = u, *b = v, *c = w;
+    for (int k = 0; k < 3; ++k) {
+        auto args = make_args<double, double>(g, a, b, c, nullptr, sfs, mu, rho);
+        double* out = st + 3 * d.n * k;
+        const cudaError_t e = stage<double, double, kModeState>(
+            "rhs_state_f64", d, args, (double*)u, (double*)v, (double*)w, out, (double*)nullptr,
+            0.5 * dt, 0.0, s);
+        if (e != cudaSuccess) return e;
+        a = out; b = out + d.n; c = out + 2 * d.n;
+    }
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

@@ -124,3 +124,33 @@ def test_sfs_stress_gradient_vs_finite_differences(A):
     fd = (Lof(eps) - Lof(-eps)) / (2 * eps)
     ad = float((F.grad * dF).sum())
     assert abs(fd - ad) <= 1e-5 * abs(ad), (fd, ad)
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 5), (7, 9, 33), (16, 20, 12)])
+@pytest.mark.parametrize("rk4,with_sfs", [(True, True), (True, False), (False, True)])
+def test_predictor_vjp_is_the_composed_stages(A, shape, rk4, with_sfs):
+    """pf_predictor_vjp against the reversed stages composed from rhs_adjoint
+    and sfs_adjoint_accumulate with torch: bit for bit (the same operations,
+    each rounded once)."""
+    rng = np.random.default_rng(7)
+    sp = (0.31, 0.17, 0.23)
+    mu, rho, dt = 0.013, 1.2, 0.01
+    r = lambda *s: torch.tensor(rng.standard_normal(s), device="cuda")  # noqa: E731
+    state, lam = [r(*shape) for _ in range(3)], [r(*shape) for _ in range(3)]
+    sfs = r(6, *shape) if with_sfs else None
+    out, F = A.predictor_vjp(state, lam, sp, mu, rho, dt, sfs, rk4)
+    stages = A.stage_states(state, sp, mu, rho, dt, sfs, rk4)
+    wts = (dt / 6.0, dt / 3.0, dt / 3.0, dt / 6.0) if rk4 else (dt,)
+    total, m, want = list(lam), None, torch.zeros((6,) + shape, dtype=torch.float64, device="cuda")
+    for s in reversed(range(len(stages))):
+        kbar = tuple(wts[s] * t for t in lam)
+        if m is not None:
+            kbar = tuple(a + 0.5 * dt * b for a, b in zip(kbar, m))
+        m = A.rhs_adjoint(stages[s], kbar, sp, mu, rho)
+        A.sfs_adjoint_accumulate(kbar, sp, 1.0, want)
+        total = [a + b for a, b in zip(total, m)]
+    for x, y in zip(out, total):
+        assert torch.equal(x, y)
+    assert (F is None) == (sfs is None)
+    if F is not None:
+        assert torch.equal(F, want)
