@@ -1496,9 +1496,10 @@ mg_update(Dims d, BicgScalars* sc, double* part, float* e, const float* ph,
 __global__ void __launch_bounds__(kBlock)
 mg_init(Dims d, BicgScalars* sc, double* part, const double* __restrict__ r,
         float* res, float* res0, float* e, float* p0, float* p1, float* v,
-        int max_it, double tol, double outer_tol) {
+        int max_it, double tol, double outer_tol, int gated) {
     pdl_wait();
     __shared__ double sh[32];
+    if (gated && !sc->done) return;  // the pass begun earlier goes on
     const double inv = sc->scale > 0.0 ? 1.0 / sc->scale : 0.0;
     double s = 0.0, m = 0.0;
     auto cell = [&](double rq) {
@@ -1853,10 +1854,11 @@ int mg_enqueue_setup(const MgPlan& P, cudaStream_t s) {
 }
 
 int mg_enqueue_init(const MgPlan& P, BicgScalars* sc, double* part, const double* rhs,
-                    double tol, int max_it, cudaStream_t s, double outer_tol) {
+                    double tol, int max_it, cudaStream_t s, double outer_tol, int gated) {
     const Dims& d = P.lv[0].d;
     PF_LAUNCH("mg_init", s, launch_pdl(mg_init, dim3(pointwise_grid(d.n)), dim3(kBlock), 0, s,
-        d, sc, part, rhs, P.res, P.res0, P.e, P.p[0], P.p[1], P.v, max_it, tol, outer_tol));
+        d, sc, part, rhs, P.res, P.res0, P.e, P.p[0], P.p[1], P.v, max_it, tol, outer_tol,
+        gated));
     return cudaGetLastError() == cudaSuccess ? PF_OK : PF_ERR_CUDA;
 }
 

@@ -80,11 +80,12 @@ int mg_inner_solve(const MgPlan& P, BicgScalars* sc, double* part,
 // Per-solve set-up kernels (the coarsest level's pseudo-inverse); enqueue
 // once before the first inner solve that uses the vectors of `region`.
 int mg_enqueue_setup(const MgPlan& P, cudaStream_t s);
-// Kernels of the inner solve, for graph capture: initialisation and one
-// iteration with parity k & 1 (kernels of a finished solve return at once).
+// Kernels of the inner solve, for graph capture: initialisation (gated: only
+// where no pass is running, sc->done != 0) and one iteration with parity k & 1
+// (kernels of a finished solve return at once).
 int mg_enqueue_init(const MgPlan& P, BicgScalars* sc, double* part,
                     const double* rhs, double tol, int max_it, cudaStream_t s,
-                    double outer_tol = 0.0);
+                    double outer_tol = 0.0, int gated = 0);
 int mg_enqueue_iteration(const MgPlan& P, BicgScalars* sc, double* part, int k,
                          cudaStream_t s, int use_cond = 0,
                          cudaGraphConditionalHandle cond = 0);

@@ -781,6 +781,7 @@ mixed_b_init(Dims d, BicgScalars* sc, double* part, const double* src,
             sc->max_b = mx; sc->scale = mx; sc->true_res = mx;
             sc->outer = 0; sc->total = 0; sc->counter = 0u;
             sc->use64 = 0; sc->prev_ratio = 2.0;
+            sc->done = 1;  // no pass is running
         }
     }
 }
@@ -822,8 +823,9 @@ struct PhaseResidual {
 __global__ void __launch_bounds__(kBlock, 2)
 mixed_residual(Dims d, Tiling tl, LapCoef<double> cf, BicgScalars* sc,
                double* part, const double* __restrict__ b,
-               const double* __restrict__ x, double* __restrict__ r) {
+               const double* __restrict__ x, double* __restrict__ r, int gated = 0) {
     __shared__ double sh[32];
+    if (gated && !sc->done) return;  // the pass is still running
     PhaseResidual ph{x, b, r, 0.0};
     sweep<double>(d, tl, cf, ph);
     const double bm = block_max<kBlock>(ph.mx, sh);
@@ -1731,9 +1733,12 @@ int project_solve(const pf_grid* g, double* u, double* v, double* w, double* DP,
 // the host-driven solve's rules: an FP32 pass that ended non-finite or in
 // breakdown was discarded (its fold skipped) and the solve continues with
 // FP64 passes, as it does once two FP32 passes in a row gain less than 2x.
+// gated: nothing while the pass is running, and FP64 passes are left to the
+// IF node of handle if64.
 __global__ void mixed_control(BicgScalars* sc, double min_res, int max_outer,
-                              int max_it, cudaGraphConditionalHandle cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+                              int max_it, cudaGraphConditionalHandle cond, int gated = 0,
+                              cudaGraphConditionalHandle if64 = 0) {
+    if (threadIdx.x != 0 || blockIdx.x != 0 || (gated && !sc->done)) return;
     sc->outer += 1;
     sc->total += sc->iter;
     // max|b| == 0: nothing to solve; a NaN max|b| gives a NaN ratio
@@ -1752,7 +1757,9 @@ __global__ void mixed_control(BicgScalars* sc, double min_res, int max_outer,
         sc->prev_ratio = ratio;
     }
     sc->max_res = ratio;
-    if (stop) cudaGraphSetConditional(cond, 0);
+    const bool leave = gated && !stop && sc->use64;
+    if (stop || leave) cudaGraphSetConditional(cond, 0);
+    if (leave) cudaGraphSetConditional(if64, 1);
 }
 
 // Start of a refinement pass: choose the FP64 or the FP32 pass.
@@ -1772,7 +1779,9 @@ __global__ void pass_tol64(BicgScalars* sc, double min_res) {
 // x += scale * e of the pass just run (its precision is sc->use64); an FP32
 // pass that ended non-finite or in breakdown is discarded.
 __global__ void __launch_bounds__(kBlock)
-fold_mixed(Dims d, const BicgScalars* sc, const float* e32, const double* e64, double* x) {
+fold_mixed(Dims d, const BicgScalars* sc, const float* e32, const double* e64, double* x,
+           int gated = 0) {
+    if (gated && !sc->done) return;  // the pass is still running
     const bool f64 = sc->use64 != 0;
     if (!f64 && (sc->status == PF_NONFINITE || sc->status == PF_BREAKDOWN)) return;
     if (f64 && sc->status == PF_NONFINITE) return;
@@ -2088,8 +2097,6 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
                 pass_tol64<<<1, 32, 0, cs>>>(sc, min_res);
                 bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64,
                                                                   e64);
-            } else if (mg.L) {
-                mg_enqueue_init(mg, sc, part, P.rr, kInnerTol, max_it, cs, min_res);
             } else {
                 bicg_init<float, true><<<gp, kBlock, 0, cs>>>(d, sc, part, P.rr, 0.0, 0.0, P.v32,
                                                              P.e32, max_it, kInnerTol);
@@ -2107,10 +2114,6 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
                                                                  hp);
                 bicg_ca<double><<<tiled_grid(ta64), blk2, 0, cs>>>(d, ta64, cf64, sc, part, v64,
                                                                   e64, 1, hp);
-            } else if (mg.L) {
-                // two iterations per pass of the body: the p buffers alternate
-                mg_enqueue_iteration(mg, sc, part, 0, cs, 1, hp);
-                mg_enqueue_iteration(mg, sc, part, 1, cs, 1, hp);
             } else {
                 bicg_b<float><<<tiled_grid(tb), blk2, 0, cs>>>(d, tb, cf, sc, part, P.v32, 1, hp);
                 bicg_ca<float><<<tiled_grid(ta), blk2, 0, cs>>>(d, ta, cf, sc, part, P.v32,
@@ -2118,10 +2121,56 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
             }
             return capture_end(cs, &inner_body);
         };
-        cudaGraphNode_t bif, b3;
+        // The refinement loop with FP64 passes in graph `lg` (body of a WHILE
+        // whose handle is `lh`): pass, fold, residual, control.
+        auto add_loop = [&](cudaGraph_t lg, cudaGraphConditionalHandle lh, cudaGraphNode_t np) -> int {
+            cudaGraph_t post = nullptr;
+            cudaGraphNode_t b3;
+            int rc = capture_begin(cs, nullptr);
+            if (rc) return rc;
+            fold_mixed<<<gp, kBlock, 0, cs>>>(d, sc, ecorr, e64, DP);
+            mixed_residual<<<tiled_grid(tld), blk2, 0, cs>>>(d, tld, cfd, sc, part, P.bb, DP, P.rr);
+            mixed_control<<<1, 32, 0, cs>>>(sc, min_res, 40, max_it, lh);
+            if ((rc = capture_end(cs, &post))) return rc;
+            rc = add_child(lg, np, post, &b3);
+            cudaGraphDestroy(post);
+            return rc;
+        };
+        cudaGraphNode_t np;
         if (P.sp.on) {
             // behind the direct solve only FP64 passes make sense
-            if ((rc = add_pass(body, true, &bif))) return rc;
+            if ((rc = add_pass(body, true, &np)) || (rc = add_loop(body, h, np))) return rc;
+        } else if (mg.L) {
+            // One loop for passes and iterations: each turn starts a pass if none
+            // is running, runs two iterations (the p buffers alternate), and ends
+            // the pass if it has stopped; kernels whose turn it is not return at
+            // once (1 us each).  Against the iterations as a WHILE node in an IF
+            // node in the passes' WHILE node, the conditional nodes saved outweigh
+            // those: ten 32^3 steps 5.88 ms against 6.02, an ensemble with one such
+            // member 8.62 against 8.76 (four steps).  FP64 passes, rare, sit behind
+            // the loop in an IF node.
+            cudaGraphConditionalHandle hif;
+            if (cudaGraphConditionalHandleCreate(&hif, C, 0, cudaGraphCondAssignDefault) != cudaSuccess)
+                return PF_ERR_CUDA;
+            if ((rc = capture_begin(cs, body))) return rc;
+            mg_enqueue_init(mg, sc, part, P.rr, kInnerTol, max_it, cs, min_res, 1);
+            mg_enqueue_iteration(mg, sc, part, 0, cs);
+            mg_enqueue_iteration(mg, sc, part, 1, cs);
+            fold_mixed<<<gp, kBlock, 0, cs>>>(d, sc, ecorr, e64, DP, 1);
+            mixed_residual<<<tiled_grid(tld), blk2, 0, cs>>>(d, tld, cfd, sc, part, P.bb, DP, P.rr, 1);
+            mixed_control<<<1, 32, 0, cs>>>(sc, min_res, 40, max_it, h, 1, hif);
+            if ((rc = capture_end(cs, &body))) return rc;
+            cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
+            prm.conditional.handle = hif;
+            prm.conditional.type = cudaGraphCondTypeIf;
+            prm.conditional.size = 1;
+            if (cudaGraphAddNode(&nsolved, C, &nw, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
+            cudaGraph_t lg, if_body = prm.conditional.phGraph_out[0];
+            cudaGraphConditionalHandle lh;
+            cudaGraphNode_t nl;
+            if ((rc = add_while(if_body, nullptr, &nl, &lg, &lh)) || (rc = add_pass(lg, true, &np)) ||
+                (rc = add_loop(lg, lh, np)))
+                return rc;
         } else {
             // outer body: branch kernel, IF(use64) {FP64 pass} ELSE {FP32 pass},
             // then fold + residual + control
@@ -2137,19 +2186,11 @@ static int add_solve_chain(cudaGraph_t G, cudaGraphNode_t dep, const pf_grid* g,
             prm.conditional.handle = hif;
             prm.conditional.type = cudaGraphCondTypeIf;
             prm.conditional.size = 2;
-            if (cudaGraphAddNode(&bif, body, &b0, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
-            if ((rc = add_pass(prm.conditional.phGraph_out[1], false, &cw))) return rc;
-            if ((rc = add_pass(prm.conditional.phGraph_out[0], true, &cw))) return rc;
+            if (cudaGraphAddNode(&np, body, &b0, 1, &prm) != cudaSuccess) return PF_ERR_CUDA;
+            if ((rc = add_pass(prm.conditional.phGraph_out[1], false, &cw)) ||
+                (rc = add_pass(prm.conditional.phGraph_out[0], true, &cw)) || (rc = add_loop(body, h, np)))
+                return rc;
         }
-        cudaGraph_t post = nullptr;
-        if ((rc = capture_begin(cs, nullptr))) return rc;
-        fold_mixed<<<gp, kBlock, 0, cs>>>(d, sc, ecorr, e64, DP);
-        mixed_residual<<<tiled_grid(tld), blk2, 0, cs>>>(d, tld, cfd, sc, part, P.bb, DP, P.rr);
-        mixed_control<<<1, 32, 0, cs>>>(sc, min_res, 40, max_it, h);
-        if ((rc = capture_end(cs, &post))) return rc;
-        rc = add_child(body, bif, post, &b3);
-        cudaGraphDestroy(post);
-        if (rc) return rc;
     }
     cudaGraphNode_t last;
     return add_step_end(C, nsolved, g, P, u, v, w, p, DP, rho, dt, prec != PF_FP64, stats, cs,
