@@ -32,6 +32,7 @@ struct RhsArgs {
     const T* visc;  // nullptr: constant mu
     const T* sfs;   // nullptr or FXX,FYY,FZZ,FXY,FXZ,FYZ
     T mu, rho, dxi, dyi, dzi;
+    int vec;        // rows of u, v, w consist of 16-byte aligned chunks
 };
 
 
@@ -130,23 +131,64 @@ rhs_stage_kernel(Dims d, RhsArgs<T, TI> a, double* __restrict__ u,
 // Tiled form (constant viscosity, no SFS stresses: the DNS hot path).  A block
 // of 32 x 8 threads owns a 32 (z) x 16 (y) tile and marches along x.  The
 // velocity of planes i-1, i, i+1 (with a one-cell y/z halo, corners included)
-// sits in a four-slot ring in shared memory; while plane i is computed,
-// cp.async copies plane i+2 into the free slot and the per-cell stage inputs
-// of plane i+1 (u, v, w and the k-sum) into a second buffer, so no thread
-// waits on global memory inside the march and no registers hold the
-// prefetch.  Every global value is read once per tile; the flux arithmetic
-// is rhs_core, unchanged.
+// sits in a four-slot ring in shared memory.  One barrier per plane, between
+// the face terms and their assembly: it publishes plane i+2, copied by cp.async
+// since the last one, and frees plane i-1's slot for plane i+3.  Every global
+// value is read once per tile; the flux arithmetic is rhs_core, unchanged.
+//
+// Bound by issue slots and the shared-memory pipe at two blocks per SM, not by
+// DRAM (63 bytes per cell and stage).  A 32-lane cp.async of 4 bytes costs four
+// shared-memory wavefronts, one of 16 bytes little more, so planes are copied
+// in 16-byte chunks where rows are aligned, and the stage inputs of FP32 stages
+// (u, v, w and the k-sum of the owned cells) go to registers, loaded before the
+// plane is computed.  Four FP32 stages, against single-element copies of planes
+// and stage inputs and a second barrier: 155 -> 138 us at 128^3, 8.30 -> 7.16 ms
+// at 512^3 (chunks and registers 147 us / 7.63 ms, the barrier the rest).  Three
+// blocks per SM spill (191 us); two rows to a packed f32x2 register are slower
+// (167 us: the FP32 pipe does not get faster) and not bitwise (the assembler
+// fuses mul.rn.f32x2 and add).
 // ---------------------------------------------------------------------------
 constexpr int kRhsTY = 16;
-constexpr int kRhsSY = kRhsTY + 2, kRhsSZ = 34;
-constexpr int kRhsPos = kRhsSY * kRhsSZ;        // halo-extended plane tile
-constexpr int kRhsPPT = (kRhsPos + 255) / 256;  // positions per thread
+constexpr int kRhsSY = kRhsTY + 2;
 constexpr int kRhsCells = 32 * kRhsTY;          // owned cells per plane
+
+// Halo-extended plane tile of elements T: rows of 32 columns with a whole
+// 16-byte chunk on either side, so that a plane whose rows are aligned is
+// copied in 16-byte pieces (column -1 is the last element of its chunk).
+template <typename T>
+struct RhsRow {
+    static constexpr int kCh = 16 / (int)sizeof(T);              // elements per chunk
+    static constexpr int kPitch = 32 + 2 * kCh;
+    static constexpr int kPos = kRhsSY * kPitch;                 // elements per plane tile
+    static constexpr int kChunks = kPos / kCh;
+    static constexpr int kPer = (kChunks + 255) / 256;           // chunks per thread
+    static constexpr int kOne = (kRhsSY * 34 + 255) / 256;       // single positions per thread
+    static __device__ __forceinline__ int at(int row, int col) { return (row + 1) * kPitch + col + kCh; }
+};
+
+// x planes per tile of a launch: the split with the least time by the model
+// waves x (planes + 2), the start-up of a march (three planes loaded before the
+// first is computed, its x-minus faces) counted as two planes.  Any split gives
+// the same bits.
+static Tiling rhs_tiling(const Dims& d) {
+    Tiling t = make_tiling(d, kRhsTY);
+    const long long yz = (long long)t.ntz * t.nty, slots = (long long)num_sms() * 2;
+    double best = 1e300;
+    for (int xc = std::min(d.nx, 2); xc <= std::min(d.nx, 128); ++xc) {
+        const long long n = (d.nx + xc - 1) / xc;
+        const double c = double((yz * n + slots - 1) / slots) * (xc + 2);
+        if (c < best) { best = c; t.xc = xc; t.ntx = (int)n; }
+    }
+    t.ntiles = yz * t.ntx;
+    return t;
+}
 
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    if (BYTES == 8)
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(s), "l"(gmem) : "memory");
+    else if (BYTES == 8)
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(s), "l"(gmem) : "memory");
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(s), "l"(gmem) : "memory");
@@ -167,14 +209,16 @@ struct RhsSmem {
     static constexpr bool kU = MODE == kModeFirst || MODE == kModeMid || MODE == kModeLast ||
                                MODE == kModeState;
     static constexpr bool kA = MODE == kModeMid || MODE == kModeLast;
-    static constexpr size_t kEu = (kU && !kConv) ? 2 * 3 * kRhsCells * sizeof(double) : 0;  // [2][3][cells]
-    static constexpr size_t kStg = kConv ? 4 * 3 * kRhsPos * sizeof(TI) : 0;             // [4][3][pos]
-    static constexpr size_t kRing = 4 * 3 * kRhsPos * (kConv ? sizeof(T) : sizeof(TI)); // [4][3][pos]
-    static constexpr size_t kEa = kA ? 2 * 3 * kRhsCells * sizeof(TA) : 0;               // [2][3][cells]
-    // y-plus terms of the rows 2 ty - 1 (8 x 32) and z-plus terms of the
-    // halo column z = -1 (16 rows) of the face form
-    static constexpr size_t kFaces = ((8 * 32 * sizeof(YFace<T>) + kRhsTY * sizeof(ZFace<T>)) + 15) &
-                                     ~size_t(15);
+    // FP64 stages keep their stage inputs in shared memory, FP32 ones in registers
+    static constexpr bool kStage = sizeof(T) == 8;
+    static constexpr size_t kEu = (kU && kStage) ? 2 * 3 * kRhsCells * sizeof(double) : 0;  // [2][3][cells]
+    static constexpr size_t kStg = kConv ? 4 * 3 * RhsRow<TI>::kPos * sizeof(TI) : 0;       // [4][3][pos]
+    static constexpr size_t kRing = 4 * 3 * RhsRow<T>::kPos * sizeof(T);                    // [4][3][pos]
+    static constexpr size_t kEa = (kA && kStage) ? 2 * 3 * kRhsCells * sizeof(TA) : 0;      // [2][3][cells]
+    // y-plus terms of the rows 2 ty - 1 (8 x 32) and z-plus terms of the halo
+    // column z = -1 (16 rows) of the face form, for two planes
+    static constexpr int kY = 8 * 32, kZ = kRhsTY;
+    static constexpr size_t kFaces = 2 * (kY * sizeof(YFace<T>) + kZ * sizeof(ZFace<T>));
     static constexpr size_t bytes = kEu + kStg + kRing + kEa + kFaces;
 };
 
@@ -186,20 +230,68 @@ __device__ __forceinline__ ZFace<T> shfl_up_z(const ZFace<T>& z) {
                     __shfl_up_sync(m, z.cvw, 1), __shfl_up_sync(m, z.cww, 1)};
 }
 
-template <typename T, typename TI>
+template <typename T>
 struct SmemSrc {
-    const TI* ring;  // [4][3][kRhsPos]
+    const T* ring;   // [4][3][pos]
     int s0, s1, s2;  // slots of planes i-1, i, i+1
-    int y, z;        // the cell in the halo-extended tile
-    __device__ const TI* f(int fld, int di) const {
+    int o;           // the cell's position in the plane tile
+    __device__ T at(int fld, int di, int dj, int dk) const {
         const int sl = di < 0 ? s0 : (di == 0 ? s1 : s2);
-        return ring + (sl * 3 + fld) * kRhsPos;
+        return ring[(sl * 3 + fld) * RhsRow<T>::kPos + o + dj * RhsRow<T>::kPitch + dk];
     }
-    __device__ T u(int di, int dj, int dk) const { return T(f(0, di)[(y + dj) * kRhsSZ + z + dk]); }
-    __device__ T v(int di, int dj, int dk) const { return T(f(1, di)[(y + dj) * kRhsSZ + z + dk]); }
-    __device__ T w(int di, int dj, int dk) const { return T(f(2, di)[(y + dj) * kRhsSZ + z + dk]); }
-    __device__ T visc(int, int, int) const { return T(0); }
-    __device__ T sfs(int, int, int, int) const { return T(0); }
+    __device__ T u(int di, int dj, int dk) const { return at(0, di, dj, dk); }
+    __device__ T v(int di, int dj, int dk) const { return at(1, di, dj, dk); }
+    __device__ T w(int di, int dj, int dk) const { return at(2, di, dj, dk); }
+};
+
+// This thread's share of a plane tile copied by cp.async: chunks, or single
+// elements where rows are not aligned.
+template <typename TI>
+struct PlaneCopy {
+    using Row = RhsRow<TI>;
+    int g[Row::kOne], o[Row::kOne];  // offset in the plane, position in the tile (-1: none)
+    bool vec;
+    __device__ PlaneCopy(const Dims& d, int j0, int k0, bool vec_) : vec(vec_) {
+        const int tid = threadIdx.y * 32 + threadIdx.x;
+        const int w = vec ? Row::kPitch / Row::kCh : 34, e = vec ? Row::kCh : 1;
+#pragma unroll
+        for (int p = 0; p < Row::kOne; ++p) {
+            const int q = tid + 256 * p, r = q / w, c = q - r * w;
+            const int col = vec ? (c - 1) * e : c - 1;
+            const bool in = r < kRhsSY;
+            o[p] = in ? Row::at(r - 1, col) : -1;
+            g[p] = in ? pmod(j0 + r - 1, d.ny) * d.nz + pmod(k0 + col, d.nz) : 0;
+        }
+    }
+    __device__ __forceinline__ void load(TI* dst, const TI* src) const {
+        if (vec) {
+#pragma unroll
+            for (int p = 0; p < Row::kPer; ++p)
+                if (o[p] >= 0) cp_async<16>(dst + o[p], src + g[p]);
+        } else {
+#pragma unroll
+            for (int p = 0; p < Row::kOne; ++p)
+                if (o[p] >= 0) cp_async<sizeof(TI)>(dst + o[p], src + g[p]);
+        }
+    }
+    // the copied elements, by the thread that copied them, in another type
+    template <typename T>
+    __device__ __forceinline__ void convert(T* dst, const TI* src) const {
+        constexpr int shift = RhsRow<T>::kCh - Row::kCh, more = RhsRow<T>::kPitch - Row::kPitch;
+        if (vec) {
+#pragma unroll
+            for (int p = 0; p < Row::kPer; ++p)
+                if (o[p] >= 0) {
+                    const int x = o[p] + o[p] / Row::kPitch * more + shift;
+#pragma unroll
+                    for (int e = 0; e < Row::kCh; ++e) dst[x + e] = T(src[o[p] + e]);
+                }
+        } else {
+#pragma unroll
+            for (int p = 0; p < Row::kOne; ++p)
+                if (o[p] >= 0) dst[o[p] + o[p] / Row::kPitch * more + shift] = T(src[o[p]]);
+        }
+    }
 };
 
 // The right-hand side of this thread's two cells of plane i (rows 2 ty and
@@ -213,39 +305,39 @@ struct SmemSrc {
 // by the second warp).  Bit-identical to rhs_core (checked on the host).
 // Every thread of the block must call it (it holds a block barrier); cells
 // outside the grid compute on wrapped data and are not stored.
-template <typename T, typename TI>
+template <typename T, class Mid>
 __device__ __forceinline__ void
-rhs_plane_faces(const TI* ring, int s0, int s1, int s2, const FluxCoef<T>& fc, bool first,
-                XFace<T> (&xf)[2], YFace<T>* sY, ZFace<T>* sZh, T (&k3)[2][3]) {
+rhs_plane_faces(const T* ring, int s0, int s1, int s2, const FluxCoef<T>& fc, bool first,
+                XFace<T> (&xf)[2], YFace<T>* sY, ZFace<T>* sZh, T (&k3)[2][3], Mid mid) {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     PlusFaces<T> pf[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-        const SmemSrc<T, TI> src{ring, s0, s1, s2, 2 * ty + r + 1, tx + 1};
+        const SmemSrc<T> src{ring, s0, s1, s2, RhsRow<T>::at(2 * ty + r, tx)};
         pf[r] = plus_faces<T>(src, fc);
     }
     if (ty < 7) sY[(ty + 1) * 32 + tx] = pf[1].y;
     if (tid < 32) {            // row -1: its y-plus terms are the y-minus terms of row 0
-        const SmemSrc<T, TI> src{ring, s0, s1, s2, 0, tid + 1};
+        const SmemSrc<T> src{ring, s0, s1, s2, RhsRow<T>::at(-1, tid)};
         sY[tid] = plus_faces<T, false, true, false>(src, fc).y;
     } else if (tid < 32 + kRhsTY) {  // column z = -1: z-plus terms for lane 0
         const int row = tid - 32;
-        const SmemSrc<T, TI> src{ring, s0, s1, s2, row + 1, 0};
+        const SmemSrc<T> src{ring, s0, s1, s2, RhsRow<T>::at(row, -1)};
         sZh[row] = plus_faces<T, false, false, true>(src, fc).z;
     }
     XFace<T> xm[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         if (first) {
-            const SmemSrc<T, TI> src{ring, s0, s1, s2, 2 * ty + r + 1, tx + 1};
-            const Shifted<SmemSrc<T, TI>> prev{src, -1, 0, 0};
+            const SmemSrc<T> src{ring, s0, s1, s2, RhsRow<T>::at(2 * ty + r, tx)};
+            const Shifted<SmemSrc<T>> prev{src, -1, 0, 0};
             xm[r] = plus_faces<T, true, false, false>(prev, fc).x;
         } else {
             xm[r] = xf[r];
         }
     }
     ZFace<T> zm[2] = {shfl_up_z(pf[0].z), shfl_up_z(pf[1].z)};
-    __syncthreads();
+    mid();
     if (tx == 0) {
         zm[0] = sZh[2 * ty];
         zm[1] = sZh[2 * ty + 1];
@@ -260,9 +352,9 @@ rhs_plane_faces(const TI* ring, int s0, int s1, int s2, const FluxCoef<T>& fc, b
 // Euler's k): plane x's FP64 values arrive by cp.async in stg slot
 // (x - i0 + 1) & 3, and the thread that copied a position converts it into
 // the FP32 ring slot of the same number once the copy has landed (a thread's
-// own copies need no barrier).  Plane i + 2 is converted after plane i is
-// computed, so one barrier per plane orders conversion and use; the first
-// stage's FP64 u of the owned cells comes from plane i's stg slot.
+// own copies need no barrier).  Plane i + 2 is converted before plane i's
+// barrier; the first stage's FP64 u of the owned cells comes from plane i's stg
+// slot, which plane i + 4 takes after the next barrier.
 template <typename T, typename TI, typename TS, typename TA, int MODE>
 __device__ __forceinline__ void
 rhs_tile_conv(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a,
@@ -276,7 +368,7 @@ rhs_tile_conv(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a,
     TI* stg = reinterpret_cast<TI*>(smraw);
     T* ring = reinterpret_cast<T*>(smraw + SM::kStg);
     YFace<T>* sY = reinterpret_cast<YFace<T>*>(smraw + SM::kEu + SM::kStg + SM::kRing + SM::kEa);
-    ZFace<T>* sZh = reinterpret_cast<ZFace<T>*>(sY + 8 * 32);
+    ZFace<T>* sZh = reinterpret_cast<ZFace<T>*>(sY + 2 * SM::kY);
     const FluxCoef<T> fc = flux_coef<T>(a.mu, a.rho, a.dxi, a.dyi, a.dzi);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     const long long plane = (long long)d.ny * d.nz;
@@ -290,17 +382,7 @@ rhs_tile_conv(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a,
         const int k0 = tz * 32, j0 = tyy * kRhsTY, i0 = txx * tl.xc;
         const int i1 = min(i0 + tl.xc, d.nx);
         const int ez = min(32, d.nz - k0), ey = min(kRhsTY, d.ny - j0);
-        long long goff[kRhsPPT];
-        int soff[kRhsPPT];
-        bool pv[kRhsPPT];
-#pragma unroll
-        for (int p = 0; p < kRhsPPT; ++p) {
-            const int pos = tid + 256 * p;
-            pv[p] = pos < kRhsPos;
-            const int yy = pv[p] ? pos / kRhsSZ : 0, zz = pv[p] ? pos - yy * kRhsSZ : 0;
-            goff[p] = (long long)pmod(j0 + yy - 1, d.ny) * d.nz + pmod(k0 + zz - 1, d.nz);
-            soff[p] = yy * kRhsSZ + zz;
-        }
+        const PlaneCopy<TI> copy(d, j0, k0, a.vec != 0);
         // this thread's owned cells: rows 2 ty and 2 ty + 1 of column tx
         bool cv[2];
         long long coff[2];
@@ -311,23 +393,16 @@ rhs_tile_conv(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a,
             coff[r] = (long long)(j0 + jl) * d.nz + k0 + tx;
         }
         auto slot = [&](int x) { return (x - i0 + 1) & 3; };
+        constexpr int kStgPos = RhsRow<TI>::kPos;
         auto load_stg = [&](int x) {
             const long long base = (long long)pmod(x, d.nx) * plane;
-            TI* dst = stg + slot(x) * 3 * kRhsPos;
 #pragma unroll
-            for (int f = 0; f < 3; ++f)
-#pragma unroll
-                for (int p = 0; p < kRhsPPT; ++p)
-                    if (pv[p]) cp_async<sizeof(TI)>(dst + f * kRhsPos + soff[p], fld[f] + base + goff[p]);
+            for (int f = 0; f < 3; ++f) copy.load(stg + (slot(x) * 3 + f) * kStgPos, fld[f] + base);
         };
         auto convert = [&](int x) {
-            const TI* src = stg + slot(x) * 3 * kRhsPos;
-            T* dst = ring + slot(x) * 3 * kRhsPos;
 #pragma unroll
             for (int f = 0; f < 3; ++f)
-#pragma unroll
-                for (int p = 0; p < kRhsPPT; ++p)
-                    if (pv[p]) dst[f * kRhsPos + soff[p]] = T(src[f * kRhsPos + soff[p]]);
+                copy.convert(ring + (slot(x) * 3 + f) * RhsRow<T>::kPos, stg + (slot(x) * 3 + f) * kStgPos);
         };
         load_stg(i0 - 1);
         load_stg(i0);
@@ -344,33 +419,34 @@ rhs_tile_conv(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a,
         for (int i = i0; i < i1; ++i) {
             const int c = i - i0;
             const int s0 = c & 3, s1 = (c + 1) & 3, s2 = (c + 2) & 3;
-            if (i + 2 < i1) load_stg(i + 3);
-            cp_async_commit();
             T k3[2][3];
-            rhs_plane_faces<T, T>(ring, s0, s1, s2, fc, i == i0, xf, sY, sZh, k3);
+            rhs_plane_faces<T>(ring, s0, s1, s2, fc, i == i0, xf, sY + (c & 1) * SM::kY,
+                               sZh + (c & 1) * SM::kZ, k3, [&] {
+                                   cp_async_wait_all();
+                                   if (i + 1 < i1) convert(i + 2);
+                                   __syncthreads();
+                                   if (i + 2 < i1) load_stg(i + 3);
+                                   cp_async_commit();
+                               });
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 if (!cv[r]) continue;
                 const int jl = 2 * ty + r;
                 const long long q = (long long)i * plane + coff[r];
-                const int pc = (jl + 1) * kRhsSZ + tx + 1;
+                const int pc = RhsRow<TI>::at(jl, tx);
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
                     const T kf = k3[r][f];
                     if (MODE == kModeFirst) {
                         // ZAXPY(h, k, u) = h*k + u (src/data/state.py:157-165)
-                        S[f][q] = TS(hdt * double(kf) + double(stg[(s1 * 3 + f) * kRhsPos + pc]));
+                        S[f][q] = TS(hdt * double(kf) + double(stg[(s1 * 3 + f) * kStgPos + pc]));
                         A[f][q] = TA(kf);
                     } else {  // kModeK
                         A[f][q] = TA(kf);
                     }
                 }
             }
-            cp_async_wait_groups<1>();
-            if (i + 1 < i1) convert(i + 2);
-            __syncthreads();
         }
-        cp_async_wait_all();
         __syncthreads();
     }
 }
@@ -388,7 +464,7 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
     TI* ring = reinterpret_cast<TI*>(smraw + SM::kEu);
     TA* ea = reinterpret_cast<TA*>(smraw + SM::kEu + SM::kRing);
     YFace<T>* sY = reinterpret_cast<YFace<T>*>(smraw + SM::kEu + SM::kStg + SM::kRing + SM::kEa);
-    ZFace<T>* sZh = reinterpret_cast<ZFace<T>*>(sY + 8 * 32);
+    ZFace<T>* sZh = reinterpret_cast<ZFace<T>*>(sY + 2 * SM::kY);
     const FluxCoef<T> fc = flux_coef<T>(a.mu, a.rho, a.dxi, a.dyi, a.dzi);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     const long long plane = (long long)d.ny * d.nz;
@@ -403,17 +479,7 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
         const int k0 = tz * 32, j0 = tyy * kRhsTY, i0 = txx * tl.xc;
         const int i1 = min(i0 + tl.xc, d.nx);
         const int ez = min(32, d.nz - k0), ey = min(kRhsTY, d.ny - j0);
-        long long goff[kRhsPPT];
-        int soff[kRhsPPT];
-        bool pv[kRhsPPT];
-#pragma unroll
-        for (int p = 0; p < kRhsPPT; ++p) {
-            const int pos = tid + 256 * p;
-            pv[p] = pos < kRhsPos;
-            const int yy = pv[p] ? pos / kRhsSZ : 0, zz = pv[p] ? pos - yy * kRhsSZ : 0;
-            goff[p] = (long long)pmod(j0 + yy - 1, d.ny) * d.nz + pmod(k0 + zz - 1, d.nz);
-            soff[p] = yy * kRhsSZ + zz;
-        }
+        const PlaneCopy<TI> copy(d, j0, k0, a.vec != 0);
         // this thread's owned cells: rows 2 ty and 2 ty + 1 of column tx
         bool cv[2];
         long long coff[2];
@@ -426,14 +492,12 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
         auto load_plane = [&](int x, int slot) {
             const long long base = (long long)pmod(x, d.nx) * plane;
 #pragma unroll
-            for (int f = 0; f < 3; ++f)
-#pragma unroll
-                for (int p = 0; p < kRhsPPT; ++p)
-                    if (pv[p])
-                        cp_async<sizeof(TI)>(ring + (slot * 3 + f) * kRhsPos + soff[p],
-                                             fld[f] + base + goff[p]);
+            for (int f = 0; f < 3; ++f) copy.load(ring + (slot * 3 + f) * RhsRow<T>::kPos, fld[f] + base);
         };
+        // stage inputs of plane x: FP64 stages copy them a plane ahead, FP32
+        // stages load them into registers before the plane is computed
         auto load_epi = [&](int x, int buf) {
+            if (!SM::kStage) return;
             const long long base = (long long)x * plane;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -447,26 +511,42 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
                 }
             }
         };
-        // prologue: planes i0-1, i0, i0+1 into slots 0, 1, 2; stage inputs of i0
+        // prologue: planes i0-1, i0, i0+1 into slots 0, 1, 2
         load_plane(i0 - 1, 0);
         load_plane(i0, 1);
         load_plane(i0 + 1, 2);
+        cp_async_commit();
+        if (i0 + 1 < i1) load_plane(i0 + 2, 3);
         load_epi(i0, 0);
         cp_async_commit();
-        cp_async_wait_all();
+        cp_async_wait_groups<1>();
         __syncthreads();
         XFace<T> xf[2];  // x-plus terms of this thread's two cells on the previous plane
         for (int i = i0; i < i1; ++i) {
             const int c = i - i0;
             const int s0 = c & 3, s1 = (c + 1) & 3, s2 = (c + 2) & 3;
             const int buf = c & 1;
-            if (i + 1 < i1) {
-                load_plane(i + 2, (c + 3) & 3);
-                load_epi(i + 1, buf ^ 1);
-                cp_async_commit();
+            double ru[2][3];
+            TA ra[2][3];
+            if (!SM::kStage) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int f = 0; f < 3; ++f) {
+                        const long long q = (long long)i * plane + coff[r];
+                        if (SM::kU) ru[r][f] = cv[r] ? U[f][q] : 0.0;
+                        if (SM::kA) ra[r][f] = cv[r] ? A[f][q] : TA(0);
+                    }
             }
             T k3[2][3];
-            rhs_plane_faces<T, TI>(ring, s0, s1, s2, fc, i == i0, xf, sY, sZh, k3);
+            rhs_plane_faces<T>(ring, s0, s1, s2, fc, i == i0, xf, sY + (c & 1) * SM::kY,
+                               sZh + (c & 1) * SM::kZ, k3, [&] {
+                                   cp_async_wait_all();
+                                   __syncthreads();
+                                   if (i + 2 < i1) load_plane(i + 3, s0);
+                                   if (i + 1 < i1) load_epi(i + 1, buf ^ 1);
+                                   cp_async_commit();
+                               });
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 if (!cv[r]) continue;
@@ -476,22 +556,24 @@ rhs_tile(const Dims& d, const Tiling& tl, const RhsArgs<T, TI>& a, double* __res
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
                     const T kf = k3[r][f];
+                    double us = 0.0;
+                    TA as = TA(0);
+                    if (SM::kU) us = SM::kStage ? eu[(buf * 3 + f) * kRhsCells + cc] : ru[r][f];
+                    if (SM::kA) as = SM::kStage ? ea[(buf * 3 + f) * kRhsCells + cc] : ra[r][f];
                     if (MODE == kModeFirst || MODE == kModeMid || MODE == kModeState) {
                         // ZAXPY(h, k, u) = h*k + u (src/data/state.py:157-165)
-                        S[f][q] = TS(hdt * double(kf) + eu[(buf * 3 + f) * kRhsCells + cc]);
+                        S[f][q] = TS(hdt * double(kf) + us);
                         if (MODE == kModeFirst) A[f][q] = TA(kf);
-                        else if (MODE == kModeMid) A[f][q] = TA(T(ea[(buf * 3 + f) * kRhsCells + cc]) + T(2.0) * kf);
+                        else if (MODE == kModeMid) A[f][q] = TA(T(as) + T(2.0) * kf);
                     } else if (MODE == kModeLast) {
-                        U[f][q] = eu[(buf * 3 + f) * kRhsCells + cc] +
-                                  c6 * (double(T(ea[(buf * 3 + f) * kRhsCells + cc]) + kf));
+                        U[f][q] = us + c6 * (double(T(as) + kf));
                     } else {  // kModeK
                         A[f][q] = TA(kf);
                     }
                 }
             }
-            cp_async_wait_all();
-            __syncthreads();
         }
+        __syncthreads();
     }
 }
 
@@ -626,6 +708,8 @@ static RhsArgs<T, TI> make_args(const pf_grid* g, const TI* u, const TI* v,
     a.u = u; a.v = v; a.w = w; a.visc = visc; a.sfs = sfs;
     a.mu = T(mu); a.rho = T(rho);
     a.dxi = T(1.0 / g->dx); a.dyi = T(1.0 / g->dy); a.dzi = T(1.0 / g->dz);
+    a.vec = g->nz % (16 / (int)sizeof(TI)) == 0 &&
+            (((uintptr_t)u | (uintptr_t)v | (uintptr_t)w) & 15) == 0;
     return a;
 }
 
@@ -663,7 +747,7 @@ static cudaError_t stage(const char* name, const Dims& d, const RhsArgs<T, TI>& 
     T* sw = st ? st + 2 * n : nullptr;
     dim3 blk(32, 8);
     if (!a.visc && !a.sfs) {
-        const Tiling tl = make_tiling(d, kRhsTY);
+        const Tiling tl = rhs_tiling(d);
         const cudaError_t e = tiled_prepare<T, TI, MODE>();
         if (e != cudaSuccess) return e;
         PF_LAUNCH(name, s, rhs_stage_tiled<T, TI, T, T, MODE><<<tiled_grid(tl), blk,
