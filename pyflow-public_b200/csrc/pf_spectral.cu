@@ -22,129 +22,18 @@
 // element-wise accesses conflict.  A thread holds 8 complex values.  In the x
 // and y passes a line pair is two neighbouring cells in z, and a block's L = 8
 // pairs read and write runs of 128 bytes; in the z pass the rows themselves
-// are contiguous.
+// are contiguous.  Extents 2^k, 3 2^k and 5 2^k from 32 to 1024 have kernels of
+// their own (pf_spectral_fast.cu).
 #include <algorithm>
 #include <cmath>
 
 #include "pf_common.cuh"
 #include "pf_kernels.cuh"
 #include "pf_profile.cuh"
-#include "pf_spectral.cuh"
+#include "pf_spectral_pass.cuh"
 
 namespace pf {
 namespace {
-
-enum { kPassZ = 0, kPassY = 1, kPassX = 2 };
-constexpr int kHold = 8;          // complex values a thread holds
-constexpr int kMaxThreads = 512;
-
-struct PassArgs {
-    SpectralAxis ax;
-    const double* src;
-    double* dst;
-    long long nlines;   // real lines in all (z: rows; x: ny nz), or nz per i (y)
-    long long stride;   // distance of consecutive elements of a line
-    int tiles;          // y: tiles per x plane
-    int vec;            // pairs of cells are 16-byte aligned
-    // x pass
-    double scale;       // c / (nx ny nz)
-    const double *lamy, *lamz;
-    int nz;
-    int* nonfin;        // first z pass: set where the input is not finite
-};
-
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
-}
-
-// Forward DFT of R values in place.
-template <int R>
-struct Dft {
-    // odd R: the terms j and R - j share their products
-    static __device__ __forceinline__ void run(double2* a) {
-        // cos, sin(2 pi m / R), m = 1 .. (R-1)/2
-        constexpr double c3[1] = {-0.5}, s3[1] = {0.86602540378443864676};
-        constexpr double c5[2] = {0.30901699437494742410, -0.80901699437494742410};
-        constexpr double s5[2] = {0.95105651629515357212, 0.58778525229247312917};
-        constexpr double c7[3] = {0.62348980185873353053, -0.22252093395631440429,
-                                  -0.90096886790241912624};
-        constexpr double s7[3] = {0.78183148246802980871, 0.97492791218182360702,
-                                  0.43388373911755812048};
-        constexpr int H = (R - 1) / 2;
-        double2 t[H], u[H];
-        double2 y0 = a[0];
-#pragma unroll
-        for (int j = 0; j < H; ++j) {
-            t[j] = cadd(a[j + 1], a[R - 1 - j]);
-            u[j] = csub(a[j + 1], a[R - 1 - j]);
-            y0 = cadd(y0, t[j]);
-        }
-        const double2 a0 = a[0];
-        a[0] = y0;
-#pragma unroll
-        for (int k = 1; k <= H; ++k) {
-            double2 m = a0, s = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int j = 0; j < H; ++j) {
-                const int q = (j + 1) * k % R;
-                const int h = q <= H ? q - 1 : R - q - 1;
-                const double c = R == 3 ? c3[h % 1] : (R == 5 ? c5[h % 2] : c7[h % 3]);
-                const double sv = R == 3 ? s3[h % 1] : (R == 5 ? s5[h % 2] : s7[h % 3]);
-                const double sg = q <= H ? sv : -sv;
-                m.x = fma(c, t[j].x, m.x);
-                m.y = fma(c, t[j].y, m.y);
-                s.x = fma(sg, u[j].x, s.x);
-                s.y = fma(sg, u[j].y, s.y);
-            }
-            a[k] = make_double2(m.x + s.y, m.y - s.x);
-            a[R - k] = make_double2(m.x - s.y, m.y + s.x);
-        }
-    }
-};
-
-template <>
-struct Dft<2> {
-    static __device__ __forceinline__ void run(double2* a) {
-        const double2 t = csub(a[0], a[1]);
-        a[0] = cadd(a[0], a[1]);
-        a[1] = t;
-    }
-};
-
-template <>
-struct Dft<4> {
-    static __device__ __forceinline__ void run(double2* a) {
-        const double2 t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
-        const double2 t2 = cadd(a[1], a[3]), t3 = csub(a[1], a[3]);
-        a[0] = cadd(t0, t2);
-        a[2] = csub(t0, t2);
-        a[1] = make_double2(t1.x + t3.y, t1.y - t3.x);
-        a[3] = make_double2(t1.x - t3.y, t1.y + t3.x);
-    }
-};
-
-template <>
-struct Dft<8> {
-    static __device__ __forceinline__ void run(double2* a) {
-        double2 e[4] = {a[0], a[2], a[4], a[6]}, o[4] = {a[1], a[3], a[5], a[7]};
-        Dft<4>::run(e);
-        Dft<4>::run(o);
-        const double c = 0.70710678118654752440;
-        const double2 o1 = make_double2(c * (o[1].x + o[1].y), c * (o[1].y - o[1].x));
-        const double2 o2 = make_double2(o[2].y, -o[2].x);
-        const double2 o3 = make_double2(c * (o[3].y - o[3].x), -c * (o[3].x + o[3].y));
-        a[0] = cadd(e[0], o[0]); a[4] = csub(e[0], o[0]);
-        a[1] = cadd(e[1], o1);   a[5] = csub(e[1], o1);
-        a[2] = cadd(e[2], o2);   a[6] = csub(e[2], o2);
-        a[3] = cadd(e[3], o3);   a[7] = csub(e[3], o3);
-    }
-};
-
-// slot of element e of line pair l
-template <int L>
-__device__ __forceinline__ int slot(int e, int l) { return e * L + (l ^ (e & (L - 1))); }
 
 // One Stockham stage of radix R (pp: product of the earlier radices): the
 // butterfly i of a line reads elements i + q n/R, and writes (i - k) R + k + q pp
@@ -238,12 +127,6 @@ __device__ __forceinline__ void transform(double2* sm, const double2* tw, const 
         }
         pp *= R;
     }
-}
-
-// Hartley values of the pair of real lines whose DFT is Z, from z = Z[k] and
-// y = Z[n - k].
-__device__ __forceinline__ double2 hartley(double2 z, double2 y) {
-    return make_double2(0.5 * ((z.x + y.x) - (z.y - y.y)), 0.5 * ((z.y + y.y) + (z.x - y.x)));
 }
 
 template <int L, int KIND, bool ODD>
@@ -408,8 +291,6 @@ size_t pass_smem(const SpectralAxis& ax) { return (size_t)ax.n * (ax.lines + 1) 
 
 int pass_threads(const SpectralAxis& ax) { return (ax.tp * ax.lines + 31) / 32 * 32; }
 
-typedef void (*PassKernel)(PassArgs);
-
 template <int KIND, bool ODD>
 PassKernel pass_kernel_l(int lines) {
     return lines == 8 ? spectral_pass<8, KIND, ODD>
@@ -434,12 +315,13 @@ cudaError_t spectral_attributes() {
                 if (e != cudaSuccess) return e;
             }
         }
-    return cudaSuccess;
+    return spectral_fast_attributes();
 }
 
 template <int KIND>
 void launch_pass(const char* name, const PassArgs& a, long long blocks, cudaStream_t s) {
-    PF_LAUNCH(name, s, launch_pdl(pass_kernel<KIND>(a.ax), dim3((unsigned)blocks),
+    const PassKernel fast = spectral_fast_kernel(KIND, a.ax.n);
+    PF_LAUNCH(name, s, launch_pdl(fast ? fast : pass_kernel<KIND>(a.ax), dim3((unsigned)blocks),
                                   dim3(pass_threads(a.ax)), pass_smem(a.ax), s, a));
 }
 
@@ -469,6 +351,11 @@ void axis_plan(int n, SpectralAxis* ax) {
     tp = std::max(tp, (n + kHold - 1) / kHold);  // the x pass's scaling
     ax->tp = tp;
     ax->lines = 8;
+    if (spectral_fast_kernel(kPassZ, n)) {  // its own radices, 8 values a thread
+        ax->tp = n / 8;
+        ax->lines = fast_lines(n);
+        return;
+    }
     while (ax->lines > 2 && (pass_threads(*ax) > kMaxThreads || pass_smem(*ax) > 113 * 1024))
         ax->lines /= 2;
 }

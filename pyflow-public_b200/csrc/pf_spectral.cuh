@@ -11,8 +11,8 @@ constexpr int kSpectralMaxStages = 12;
 
 // The tightest relative residual the direct solve is asked for: its own
 // residual is the rounding of an FP64 transform seen through the operator
-// (measured max|b - A x| / max|b| of step right-hand sides: 32^3 2e-15,
-// 128^3 2e-14, 512^3 3e-13).  Tighter tolerances go to the iterative solve.
+// (measured max|b - A x| / max|b| of step right-hand sides: 32^3 1e-15,
+// 128^3 2.3e-14, 512^3 1.4e-13).  Tighter tolerances go to the iterative solve.
 constexpr double kSpectralMinTol = 1e-12;
 
 // One axis' transform: n = product of the radices, run in this order.

@@ -139,3 +139,21 @@ def test_plan_takes_the_correction_back(shape):
     for x, y in zip(a[:4], b[:4]):
         assert torch.isfinite(x).all()
         assert float((x - y).abs().max()) <= 1e-6 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("n", [32, 64, 96, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024])
+@pytest.mark.parametrize("rest", [(3, 5), (2, 17), (18, 4)])
+def test_unrolled_extents_match_fft(n, rest):
+    """The extents with stages laid out at compile time, in each position, with
+    unpaired, unaligned and partial line groups beside them; bounds as above."""
+    for axis in range(3):
+        shape = rest[:axis] + (n,) + rest[axis:]
+        rng = np.random.default_rng(n + axis)
+        sp = (0.31, 0.17, 0.23)
+        src = rng.standard_normal(shape)
+        src -= src.mean()
+        want = _exact(src, sp)
+        DP, _, info = _solve(torch.tensor(src, device="cuda"), sp, "fp64", flags=0x200)
+        assert info.status == 0 and info.iterations == 1 and info.max_res <= 1e-10
+        got = DP.cpu().numpy()
+        assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
