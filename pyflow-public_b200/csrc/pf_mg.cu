@@ -871,7 +871,15 @@ __device__ __forceinline__ void bottom_load_pinv(const MgBottom& P, float* sm) {
     const int last = P.nlev - 1;
     const int nc = (int)P.d[last].n;
     float* pv = sm + P.off[last] + 3 * nc;
-    for (int q = threadIdx.x; q < nc * nc; q += blockDim.x) pv[q] = __ldg(P.pinv + q);
+    for (int q = threadIdx.x; q < nc * nc; q += 4 * blockDim.x) {
+        float v[4];  // on their way together
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            v[e] = q + e * blockDim.x < nc * nc ? __ldg(P.pinv + q + e * blockDim.x) : 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (q + e * blockDim.x < nc * nc) pv[q + e * blockDim.x] = v[e];
+    }
 }
 
 // One V-cycle over the levels of P, all in this CTA's shared memory `sm`:
@@ -913,22 +921,31 @@ __device__ void bottom_cycle(const MgBottom& P, float* sm) {
     }
     // coarsest: x = A^+ b, or mean removal then Jacobi sweeps (x <-> t)
     if (P.pinv) {
-        // x = A^+ b: 16 threads per row, 16-lane shuffle reduction
+        // x = A^+ b: 16 partial sums per row, neighbouring threads on neighbouring
+        // rows (distinct banks), then their sum as a tree.  With 16 neighbouring
+        // threads per row and shuffles the reads of pv met in two banks: 3250
+        // cycles of the 27000 of a launch at 16^3 8^3 4^3, now 700.
         const int n = (int)P.d[last].n;
         const float* b = sm + P.off[last];
         float* x = sm + P.off[last] + n;
         const float* pv = sm + P.off[last] + 3 * n;
-        // whole warps take part in every pass of the loop (the bound is a
-        // multiple of 32, like the block), so the shuffles see all lanes
-        const int tot = ((16 * n + 31) / 32) * 32;
-        for (int t = tid; t < tot; t += nt) {
-            const int p = t >> 4, part = t & 15;
+        __shared__ float psum[16 * kMgPinvMax];
+        for (int t = tid; t < 16 * n; t += nt) {
+            const int part = t / n, p = t - part * n;
             float acc = 0.0f;
-            if (p < n)
-                for (int r = part; r < n; r += 16) acc = fmaf(pv[r * n + p], b[r], acc);
+            for (int r = part; r < n; r += 16) acc = fmaf(pv[r * n + p], b[r], acc);
+            psum[t] = acc;
+        }
+        __syncthreads();
+        for (int p = tid; p < n; p += nt) {
+            float a[16];
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, 16);
-            if (part == 0 && p < n) x[p] = acc;
+            for (int q = 0; q < 16; ++q) a[q] = psum[q * n + p];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < o; ++q) a[q] += a[q + o];
+            x[p] = a[0];
         }
         __syncthreads();
     } else {
@@ -1089,6 +1106,13 @@ mg_cluster(MgCluster P, const float* __restrict__ gb, float* __restrict__ gx,
         if (r < P.ns) return tab[P.toff[r] + a * P.d[r].nx + i];
         return whole0 + P.w.off[0] + a * (int)dw.n + i * plw;
     };
+    // this CTA's planes of the first level's b (one cell per thread at most:
+    // kMgClusterMax / kClusterCtas), on their way while the rest is set up
+    static_assert(kMgClusterMax <= kClusterCtas * kBottomThreads, "one cell per thread");
+    const int cells0 = P.pp[0] * P.d[0].ny * P.d[0].nz;
+    float b0 = 0.0f;
+    if (tid < cells0) b0 = gb[(long long)rank * cells0 + tid];
+    if (rank == 0) bottom_load_pinv(P.w, sm + P.whole);
     for (int r = 0; r < P.ns; ++r) {
         const int nx = P.d[r].nx, pl = P.d[r].ny * P.d[r].nz, cells = P.pp[r] * pl;
         for (int e = tid; e < 3 * nx; e += nt) {
@@ -1097,13 +1121,7 @@ mg_cluster(MgCluster P, const float* __restrict__ gb, float* __restrict__ gx,
             tab[P.toff[r] + e] = cl.map_shared_rank(sm + P.off[r] + a * cells + li * pl, owner);
         }
     }
-    {   // this CTA's planes of the first level's b
-        const int cells = P.pp[0] * P.d[0].ny * P.d[0].nz;
-        const float* src = gb + (long long)rank * cells;
-        float* b = sm + P.off[0];
-        for (int q = tid; q < cells; q += nt) b[q] = src[q];
-    }
-    if (rank == 0) bottom_load_pinv(P.w, sm + P.whole);
+    if (tid < cells0) sm[P.off[0] + tid] = b0;
     cl.sync();
     // down: pre-smooth from zero, restrict
     for (int r = 0; r < P.ns; ++r) {
