@@ -10,12 +10,13 @@ projection -- replayed as one captured CUDA graph per step (device-side
 convergence loops, no host synchronisation inside the timed region).
 
 Precision (--prec):
-  mixed_mg (default)  fluxes, RK4 stages and Krylov vectors in FP32; FP64
-                      residuals, inner products and iterative refinement to the
-                      reference's tolerance on the FP64 true residual; the FP32
-                      passes run BiCGStab right-preconditioned by one FP32
-                      geometric-multigrid V(2,2) cycle
-  mixed               the same refinement with unpreconditioned FP32 BiCGStab
+  mixed_mg (default)  fluxes and RK4 stages in FP32; the pressure equation solved
+                      directly in FP64 by fast Hartley transforms, checked by
+                      the FP64 true residual against the reference's tolerance
+                      (FP64 BiCGStab refinement where it misses it); grids of at
+                      most 32^3 cells that coarsen: FP64 refinement by FP32
+                      BiCGStab passes right-preconditioned by one V(2,2) cycle
+  mixed               the same with the direct solve at every size
   fp64                the reference's algorithm (unpreconditioned BiCGStab) in FP64
 The mixed forms also run the FP64 form from the same field for the
 workload's full step count and report its rate and the error of the mixed
@@ -73,10 +74,10 @@ METRIC = "cell-steps/s (RK4+Poisson)"
 TOL = 1e-10
 MAX_IT = 20000
 SOLVER = {
-    "mixed_mg": "bicgstab right-preconditioned by an fp32 multigrid V(2,2) cycle, "
-                "inside fp64 iterative refinement started from the previous step's DP",
-    "mixed": "fp32 bicgstab inside fp64 iterative refinement started from the previous "
-             "step's DP",
+    "mixed_mg": "direct fp64 solve by fast Hartley transforms, checked by the fp64 true "
+                "residual (fp64 bicgstab refinement where it misses the tolerance)",
+    "mixed": "direct fp64 solve by fast Hartley transforms, checked by the fp64 true "
+             "residual (fp64 bicgstab refinement where it misses the tolerance)",
     "fp64": "bicgstab (fp64, the reference's algorithm, DP = 0 at every solve)",
 }
 

@@ -68,6 +68,10 @@ def bytes_per_cell(name):
         # clears DP: 24)
         "mixed_b_init": 16, "mixed_update": 20, "mixed_residual": 24,
         "add_inplace": 24, "div_vel": 32, "vel_corr": 56, "stats": 24,
+        # direct solve: in-place FP64 passes; its check (DP, source), the
+        # projection with p += DP (DP, u, v, w, p), and both in one pass
+        "spectral_z": 16, "spectral_y": 16, "spectral_x": 16, "spectral_check": 16,
+        "project": 72, "project_check": 80,
         "laplace_apply": 16, "jacobi_sweep": 24, "jacobi_prep": 24,
         "jacobi_residual": 16,
         # x-slab BiCGStab (FP64, per interior cell): 21 field passes per
@@ -141,8 +145,7 @@ def roofline(ktimes, ncells, prec):
 
 def step_roofline(ktimes, ncells, steps, step_ms):
     """Whole-step figure: the algorithmic bytes of every full-grid launch in
-    ``steps`` steps (coarse multigrid levels, about a seventh more, are not
-    counted) over the measured step time."""
+    ``steps`` steps (coarse multigrid levels are not counted) over the measured step time."""
     peak, src = peaks()
     total = 0.0
     for name, kt in ktimes.items():
