@@ -415,8 +415,9 @@ __device__ __forceinline__ void solve_after_b(BicgScalars& S, const double* sums
 // res, pp and t in shared memory with the stencil operand and its ring of
 // neighbours, vv and x there too (up to 4 planes) or in registers.  (Spilled
 // registers are no place for it: after a barrier's acquire every reload from
-// local memory goes to L2; with 38 spilled words an iteration took 24 us.)  Only what neighbouring tiles read travels: a block publishes res, pp,
-// vv and t of its boundary cells (in the two kernels' buffer sets) and forms
+// local memory goes to L2; with 38 spilled words an iteration took 24 us.)
+// Only what neighbouring tiles read travels: a block publishes res, pp, vv and
+// t of its boundary cells (in the two kernels' buffer sets) and forms
 // the operand of its ring cells from its neighbours' published values.
 template <int XC, int PER>
 struct TileSolve {
@@ -1180,13 +1181,15 @@ static int run_iterations(const Dims& d, const LapCoef<T>& cf,
 
 // PF_MIXED_MG grids that keep the V-cycle iterations where the direct solve
 // would serve too: all that coarsen when PF_MG_COOP asks for them, and those
-// of at most 2^15 cells.  At 32^3 a captured step takes 0.62 ms with the
+// of at most 2^15 cells.  At 32^3 a captured step takes 0.57 ms with the
 // V-cycles and 0.10 ms with the direct solve, but any change of DP, however
 // small, flips roundings of the FP32 stages, and on these coarse grids (few
 // points per wave, large steps) the two solvers' trajectories part within a
-// request: after 10 steps the velocities differ by 3e-9 (by 8e-15 after the
-// first), against 6e-11 after 5 steps at 128^3 and 7e-11 after 3 at 90x77x63.
-// Requests this small keep the results they have.
+// request: after 10 steps the velocities differ by 3e-9 (2-norm; by 8e-15
+// after the first), against at most 9e-11 after 5 steps at 128^3, 1.9e-10
+// after 3 at 90x77x63 and 2e-10 in ensembles up to 192^3 after 4 (single cells
+// beside a flip at a large velocity by up to 8e-8).  Requests this small keep
+// the results they have.
 constexpr long long kDirectMinCells = 1LL << 15;
 
 static bool mg_cycles_serve(const pf_grid* g, int prec) {
