@@ -162,3 +162,31 @@ def test_mg_cooperative_path_runs(monkeypatch):
     assert kt["mg_mid_down"]["launches"] == kt["mg_mid_up"]["launches"]
     assert "mg_smooth0_pw" not in kt and "mg_prolong_smooth_pw" not in kt
     assert _true_residual(src, DP, sp) <= 1e-10
+
+
+@pytest.mark.parametrize("n,min_res,max_it", [(32, 1e-17, 60), (16, 1e-17, 40)])
+def test_captured_vcycles_leave_for_fp64_passes(n, min_res, max_it):
+    """A tolerance below FP64 rounding: the captured refinement's V-cycle
+    passes stop gaining and the step goes on with FP64 passes up to the
+    iteration limit, like the host-driven solve; a second launch of the same
+    graph begins with V-cycles again."""
+    import pyflow_b200.initial as ic
+    import pyflow_b200.ops as ops
+    from pyflow_b200.plan import StepPlan
+    sp = (2 * np.pi / n,) * 3
+    f0 = [torch.tensor(a, device="cuda") for a in ic.spectral_velocity((n,) * 3, k0=4.0, seed=9)]
+    a = [t.clone() for t in f0] + [torch.zeros_like(f0[0]), torch.zeros_like(f0[0])]
+    b = [t.clone() for t in a]
+    plan = StepPlan(*b, sp, 0.01, 1.0, 0.005, min_res=min_res, max_it=max_it, prec="mixed_mg")
+    for _ in range(2):
+        info = ops.forward_step(*a, sp, 0.01, 1.0, 0.005, min_res=min_res, max_it=max_it,
+                                prec="mixed_mg", warm=True)
+        plan.launch(1)
+        torch.cuda.synchronize()
+        st = plan.stats()
+        assert info.status != 0 and st["status"] != 0
+        assert info.max_res < 1e-13 and st["max_res"] < 1e-13
+        # both DP within 1e-13 of max|b|: 100 times that in the velocities
+        for x, y in zip(a[:3], b[:3]):
+            assert (x - y).abs().max().item() <= 1e-11 * y.abs().max().item()
+    plan.close()
