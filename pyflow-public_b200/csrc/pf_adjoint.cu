@@ -41,24 +41,25 @@ __device__ __forceinline__ void rhs_adjoint_cell(const Dims& d, const AdjArgs& A
                                                  int k, double& ru, double& rv, double& rw) {
     const double dxi = A.dxi, dyi = A.dyi, dzi = A.dzi;
     auto at = [&](const double* f, int di, int dj, int dk) -> double {
-        const double x = __ldg(f + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
-        return f == A.mu || f == A.mv || f == A.mw ? A.scale * x : x;
+        return __ldg(f + idx(d, wrap(i + di, d.nx), wrap(j + dj, d.ny), wrap(k + dk, d.nz)));
     };
+    // the adjoint, scaled (its fields may be the state's own)
+    auto adj = [&](const double* f, int di, int dj, int dk) { return A.scale * at(f, di, dj, dk); };
     // ---- convective flux adjoints (at flux position p = c + (di,dj,dk))
-    auto lamCxx = [&](int di, int dj, int dk) { return dxi * (at(A.mu, di + 1, dj, dk) - at(A.mu, di, dj, dk)); };
-    auto lamCyy = [&](int di, int dj, int dk) { return dyi * (at(A.mv, di, dj + 1, dk) - at(A.mv, di, dj, dk)); };
-    auto lamCzz = [&](int di, int dj, int dk) { return dzi * (at(A.mw, di, dj, dk + 1) - at(A.mw, di, dj, dk)); };
+    auto lamCxx = [&](int di, int dj, int dk) { return dxi * (adj(A.mu, di + 1, dj, dk) - adj(A.mu, di, dj, dk)); };
+    auto lamCyy = [&](int di, int dj, int dk) { return dyi * (adj(A.mv, di, dj + 1, dk) - adj(A.mv, di, dj, dk)); };
+    auto lamCzz = [&](int di, int dj, int dk) { return dzi * (adj(A.mw, di, dj, dk + 1) - adj(A.mw, di, dj, dk)); };
     auto lamCxy = [&](int di, int dj, int dk) {
-        return dyi * (at(A.mu, di, dj, dk) - at(A.mu, di, dj - 1, dk)) +
-               dxi * (at(A.mv, di, dj, dk) - at(A.mv, di - 1, dj, dk));
+        return dyi * (adj(A.mu, di, dj, dk) - adj(A.mu, di, dj - 1, dk)) +
+               dxi * (adj(A.mv, di, dj, dk) - adj(A.mv, di - 1, dj, dk));
     };
     auto lamCxz = [&](int di, int dj, int dk) {
-        return dzi * (at(A.mu, di, dj, dk) - at(A.mu, di, dj, dk - 1)) +
-               dxi * (at(A.mw, di, dj, dk) - at(A.mw, di - 1, dj, dk));
+        return dzi * (adj(A.mu, di, dj, dk) - adj(A.mu, di, dj, dk - 1)) +
+               dxi * (adj(A.mw, di, dj, dk) - adj(A.mw, di - 1, dj, dk));
     };
     auto lamCyz = [&](int di, int dj, int dk) {
-        return dzi * (at(A.mv, di, dj, dk) - at(A.mv, di, dj, dk - 1)) +
-               dyi * (at(A.mw, di, dj, dk) - at(A.mw, di, dj - 1, dk));
+        return dzi * (adj(A.mv, di, dj, dk) - adj(A.mv, di, dj, dk - 1)) +
+               dyi * (adj(A.mw, di, dj, dk) - adj(A.mw, di, dj - 1, dk));
     };
     // face averages of the state entering the products
     auto cu = [&](int di, int dj, int dk) { return 0.5 * (at(A.u, di + 1, dj, dk) + at(A.u, di, dj, dk)); };
@@ -91,9 +92,9 @@ __device__ __forceinline__ void rhs_adjoint_cell(const Dims& d, const AdjArgs& A
     // ---- viscous (constant viscosity): diagonal fluxes at centres
     // FX = (ux - D/3) a, FY = (vy - D/3) a, FZ = (wz - D/3) a with D = ux+vy+wz;
     // their adjoints lX = dxi (mu_u(p) - mu_u(p+x)), ...
-    auto lX = [&](int di, int dj, int dk) { return dxi * (at(A.mu, di, dj, dk) - at(A.mu, di + 1, dj, dk)); };
-    auto lY = [&](int di, int dj, int dk) { return dyi * (at(A.mv, di, dj, dk) - at(A.mv, di, dj + 1, dk)); };
-    auto lZ = [&](int di, int dj, int dk) { return dzi * (at(A.mw, di, dj, dk) - at(A.mw, di, dj, dk + 1)); };
+    auto lX = [&](int di, int dj, int dk) { return dxi * (adj(A.mu, di, dj, dk) - adj(A.mu, di + 1, dj, dk)); };
+    auto lY = [&](int di, int dj, int dk) { return dyi * (adj(A.mv, di, dj, dk) - adj(A.mv, di, dj + 1, dk)); };
+    auto lZ = [&](int di, int dj, int dk) { return dzi * (adj(A.mw, di, dj, dk) - adj(A.mw, di, dj, dk + 1)); };
     auto sx = [&](int di, int dj, int dk) {
         return A.a * (2.0 * lX(di, dj, dk) - lY(di, dj, dk) - lZ(di, dj, dk)) / 3.0;
     };
@@ -109,16 +110,16 @@ __device__ __forceinline__ void rhs_adjoint_cell(const Dims& d, const AdjArgs& A
     aw += dzi * (sz(0, 0, -1) - sz(0, 0, 0));
     // off-diagonal fluxes on edges: FXY = ((u(p+y)-u(p)) dyi + (v(p+x)-v(p)) dxi) e
     auto txy = [&](int di, int dj, int dk) {
-        return A.e * (dyi * (at(A.mu, di, dj, dk) - at(A.mu, di, dj + 1, dk)) +
-                      dxi * (at(A.mv, di, dj, dk) - at(A.mv, di + 1, dj, dk)));
+        return A.e * (dyi * (adj(A.mu, di, dj, dk) - adj(A.mu, di, dj + 1, dk)) +
+                      dxi * (adj(A.mv, di, dj, dk) - adj(A.mv, di + 1, dj, dk)));
     };
     auto txz = [&](int di, int dj, int dk) {
-        return A.e * (dzi * (at(A.mu, di, dj, dk) - at(A.mu, di, dj, dk + 1)) +
-                      dxi * (at(A.mw, di, dj, dk) - at(A.mw, di + 1, dj, dk)));
+        return A.e * (dzi * (adj(A.mu, di, dj, dk) - adj(A.mu, di, dj, dk + 1)) +
+                      dxi * (adj(A.mw, di, dj, dk) - adj(A.mw, di + 1, dj, dk)));
     };
     auto tyz = [&](int di, int dj, int dk) {
-        return A.e * (dzi * (at(A.mv, di, dj, dk) - at(A.mv, di, dj, dk + 1)) +
-                      dyi * (at(A.mw, di, dj, dk) - at(A.mw, di, dj + 1, dk)));
+        return A.e * (dzi * (adj(A.mv, di, dj, dk) - adj(A.mv, di, dj, dk + 1)) +
+                      dyi * (adj(A.mw, di, dj, dk) - adj(A.mw, di, dj + 1, dk)));
     };
     au += dyi * (txy(0, -1, 0) - txy(0, 0, 0)) + dzi * (txz(0, 0, -1) - txz(0, 0, 0));
     av += dxi * (txy(-1, 0, 0) - txy(0, 0, 0)) + dzi * (tyz(0, 0, -1) - tyz(0, 0, 0));
@@ -129,7 +130,7 @@ __device__ __forceinline__ void rhs_adjoint_cell(const Dims& d, const AdjArgs& A
     rw = aw;
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 rhs_adjoint_kernel(Dims d, AdjArgs A, double* __restrict__ ou,
                    double* __restrict__ ov, double* __restrict__ ow) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

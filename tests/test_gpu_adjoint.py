@@ -154,3 +154,23 @@ def test_predictor_vjp_is_the_composed_stages(A, shape, rk4, with_sfs):
     assert (F is None) == (sfs is None)
     if F is not None:
         assert torch.equal(F, want)
+
+
+@pytest.mark.parametrize("rk4", [False, True])
+@pytest.mark.parametrize("which", [(0, 1, 2), (1, 2, 0), (0, None, None), (None, None, 1)])
+def test_predictor_vjp_of_an_adjoint_that_is_the_state(A, rk4, which):
+    """An adjoint field that is the state (the gradient of u^2 / 2), or shares
+    some of its components in any order, gives bit for bit what copies give:
+    the stage weight belongs to the adjoint alone."""
+    rng = np.random.default_rng(3)
+    shape, sp = (7, 9, 33), (0.31, 0.17, 0.23)
+    r = lambda: torch.tensor(rng.standard_normal(shape), device="cuda")  # noqa: E731
+    state = [r() for _ in range(3)]
+    lam = [r() if q is None else state[q] for q in which]
+    keep = [t.clone() for t in state]
+    out, _ = A.predictor_vjp(state, lam, sp, 0.013, 1.2, 0.01, None, rk4)
+    want, _ = A.predictor_vjp(keep, [t.clone() for t in lam], sp, 0.013, 1.2, 0.01, None, rk4)
+    for x, y in zip(out, want):
+        assert torch.equal(x, y)
+    for x, y in zip(state, keep):
+        assert torch.equal(x, y)
