@@ -248,8 +248,9 @@ int pf_sfs_adjoint(const pf_grid* g, const double* mu_u, const double* mu_v,
 /* Vector-Jacobian product of pf_predictor_step (FP64, constant viscosity, sfs
  * stresses or NULL) at the step input u, v, w: out = dL/d(u, v, w) for the
  * predictor's adjoint input lam, stage states recomputed; out_sfs (six fields,
- * or NULL) = dL/dsfs.  lam and out must not overlap.  Asynchronous; ws of
- * pf_predictor_vjp_workspace_bytes. */
+ * or NULL) = dL/dsfs.  Fields of lam may be fields of the state; outputs
+ * overlap neither them nor one another nor ws (PF_ERR_BAD_ARG), and ws does
+ * not overlap inputs.  Asynchronous; ws of pf_predictor_vjp_workspace_bytes. */
 size_t pf_predictor_vjp_workspace_bytes(const pf_grid* g);
 int pf_predictor_vjp(const pf_grid* g, int rk4, const double* u, const double* v,
                      const double* w, const double* lam_u, const double* lam_v,

@@ -259,6 +259,11 @@ extern "C" int pf_sfs_adjoint(const pf_grid* g, const double* mu_u,
     return cudaGetLastError() == cudaSuccess ? PF_OK : PF_ERR_CUDA;
 }
 
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + nb && y < x + na;
+}
+
 extern "C" size_t pf_predictor_vjp_workspace_bytes(const pf_grid* g) {
     if (!g || g->nx < 2 || g->ny < 2 || g->nz < 2) return 0;
     // three stage states, two sets of stage adjoints
@@ -278,6 +283,25 @@ extern "C" int pf_predictor_vjp(const pf_grid* g, int rk4, const double* u, cons
     using namespace pf;
     const Dims d{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
     const long long n = d.n;
+    // The stages read the state and the adjoint at neighbouring cells after
+    // outputs have been written, and the workspace holds stage states and
+    // adjoints (RK4): what is written shares memory with none of them.
+    {
+        struct Range { const void* p; size_t bytes; } r[11];
+        int outs = 0, k = 0;
+        const size_t b = (size_t)n * sizeof(double);
+        for (double* o : {out_u, out_v, out_w}) r[k++] = Range{o, b};
+        if (out_sfs) r[k++] = Range{out_sfs, 6 * b};
+        if (rk4) r[k++] = Range{ws, pf_predictor_vjp_workspace_bytes(g)};
+        outs = k;
+        for (const double* x : {u, v, w, lam_u, lam_v, lam_w}) r[k++] = Range{x, b};
+        for (int i = 0; i < outs; ++i)
+            for (int j = i + 1; j < k; ++j)
+                if (overlap(r[i].p, r[i].bytes, r[j].p, r[j].bytes)) return PF_ERR_BAD_ARG;
+        // (the stresses are read before any output is written)
+        if (rk4 && sfs && overlap(ws, pf_predictor_vjp_workspace_bytes(g), sfs, 6 * b))
+            return PF_ERR_BAD_ARG;
+    }
     cudaStream_t s = (cudaStream_t)stream;
     double* st = (double*)ws;
     double* kb[2] = {st + 9 * n, st + 12 * n};

@@ -240,3 +240,47 @@ def test_python_signatures_match_the_header():
             assert fn.restype is scalar[r[-1]], (name, fn.restype)
         checked += 1
     assert checked >= 30, checked
+
+
+def test_predictor_vjp_refuses_overlapping_outputs():
+    """pf_predictor_vjp reads the state and the adjoint at neighbouring cells
+    after it has written part of its outputs: an output that shares memory
+    with them, with another output or with the workspace (which the Euler form
+    does not use), or stresses in the workspace, are refused before any CUDA
+    call (the addresses here are never used).  The stresses are read before
+    any output is written: outputs may take their place."""
+    if not os.path.exists(LIB):
+        pytest.skip("library not built")
+    lib = ctypes.CDLL(LIB)
+
+    class Grid(ctypes.Structure):
+        _fields_ = [("nx", ctypes.c_int), ("ny", ctypes.c_int),
+                    ("nz", ctypes.c_int), ("dx", ctypes.c_double),
+                    ("dy", ctypes.c_double), ("dz", ctypes.c_double)]
+
+    P, D = ctypes.c_void_p, ctypes.c_double
+    fn = lib.pf_predictor_vjp
+    fn.restype = ctypes.c_int
+    fn.argtypes = [ctypes.POINTER(Grid), ctypes.c_int] + [P] * 6 + [D] * 3 + [P] * 5 + [
+        P, ctypes.c_size_t, P]
+    size = lib.pf_predictor_vjp_workspace_bytes
+    size.restype, size.argtypes = ctypes.c_size_t, [ctypes.POINTER(Grid)]
+    g = Grid(4, 3, 5, 0.1, 0.1, 0.1)
+    n, ws_bytes = 4 * 3 * 5 * 8, size(ctypes.byref(g))
+    one = 16 * n + ws_bytes
+    at = {k: one * (i + 1) for i, k in enumerate(
+        ["u", "v", "w", "lu", "lv", "lw", "sfs", "ou", "ov", "ow", "osfs", "ws"])}
+
+    def call(rk4, **moved):
+        a = dict(at, **moved)
+        return fn(ctypes.byref(g), rk4, *(a[k] for k in ("u", "v", "w", "lu", "lv", "lw")), 0.01,
+                  1.0, 0.1, a["sfs"], a["ou"], a["ov"], a["ow"], a["osfs"], a["ws"], ws_bytes, None)
+
+    for rk4 in (0, 1):
+        for k in ("u", "v", "w", "lu", "lv", "lw", "ow", "osfs"):
+            assert call(rk4, ou=at[k]) == 1, k
+            assert call(rk4, ou=at[k] + n - 8) == 1, k      # the last cell
+        for k in ("u", "lw", "ov"):
+            assert call(rk4, osfs=at[k] - 6 * n + 8) == 1, k
+    for k in ("u", "lv", "ow", "sfs", "osfs"):
+        assert call(1, ws=at[k] - ws_bytes + 8) == 1, k
