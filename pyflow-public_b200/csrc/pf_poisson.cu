@@ -1221,7 +1221,9 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
     max_it = std::max(max_it, 1);
     bool solved = false, use64 = false;
     int outer = 0, total = 0;
-    if (direct && !mg_cycles_serve(g, prec) && spectral_applies(g, min_res, DP, ptr)) {
+    // the direct solve's check reads the source again when DP is there: a DP in
+    // the source's own buffer goes to the iterations, which keep b themselves
+    if (direct && source != DP && !mg_cycles_serve(g, prec) && spectral_applies(g, min_res, DP, ptr)) {
         // the tables sit in the region of the iterative solver's vectors
         SpectralPlan sp;
         if (spectral_setup(g, ptr, &sp) != cudaSuccess ||
