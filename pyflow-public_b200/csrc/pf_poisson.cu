@@ -1235,12 +1235,19 @@ int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,
         A.min_res = min_res; A.max_it = max_it; A.DP = DP;
         launch_project<true, false>("spectral_check", g, A, s);
         if (cudaGetLastError() != cudaSuccess || read_scalars(sc, &hs, s)) return PF_ERR_CUDA;
-        solved = hs.done != 0;
-        outer = hs.max_b == 0.0 ? 0 : 1;
-        total = hs.total;
-        out.max_res = hs.max_res; out.iterations = total; out.outer = outer; out.status = hs.status;
-        // the mixed forms go on from here, in FP64; PF_FP64 starts over
-        warm = use64 = prec != PF_FP64;
+        if (hs.status == PF_NONFINITE && hs.max_b != 0.0) {
+            // a finite source (else max_b is 0 and DP was cleared) whose
+            // transforms or right-hand side overflow: the whole iterative
+            // solve, which scales its vectors, from DP = 0
+            warm = false;
+        } else {
+            solved = hs.done != 0;
+            outer = hs.max_b == 0.0 ? 0 : 1;
+            total = hs.total;
+            out.max_res = hs.max_res; out.iterations = total; out.outer = outer; out.status = hs.status;
+            // the mixed forms go on from here, in FP64; PF_FP64 starts over
+            warm = use64 = prec != PF_FP64;
+        }
     }
     if (solved) {
         // nothing more to iterate

@@ -181,3 +181,40 @@ def test_source_and_solution_in_one_buffer(prec, shape):
         assert torch.equal(p, DP)
         out.append(DP - DP.mean())
     assert float((out[0] - out[1]).norm()) <= 3e-6 * float(out[1].norm())
+
+
+@pytest.mark.parametrize("prec", ["mixed", "mixed_mg"])
+def test_sources_beyond_the_transforms_range(prec):
+    """Finite sources whose transforms overflow (their values times the square
+    root of the cells): the scaled passes solve them.  The error is at most
+    1e-10 kappa max|b| sqrt(N) / |b| of the solution (kappa 1440, 5)."""
+    shape, sp = (48, 40, 56), (0.31, 0.17, 0.23)
+    a = np.random.default_rng(2).standard_normal(shape)
+    a -= a.mean()
+    want = _exact(a, sp, 1.0, 1.0)
+    DP, p, info = _solve(torch.tensor(a * 1e307, device="cuda"), sp, prec, rho=1.0, dt=1.0)
+    assert info.status == 0 and info.max_res <= 1e-10
+    got = DP.cpu().numpy() / 1e307
+    got -= got.mean()
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+    assert torch.equal(p, 1.0 + DP)
+
+
+def test_right_hand_side_that_overflows():
+    """A finite source times an infinite rho/dt: reported, p untouched."""
+    a = np.random.default_rng(2).standard_normal((24, 20, 28))
+    src = torch.tensor(a - a.mean(), device="cuda")
+    DP, p, info = _solve(src, (0.31, 0.17, 0.23), "mixed", rho=1e200, dt=1e-200)
+    assert info.status == 5
+    assert float(DP.abs().max()) == 0.0 and torch.equal(p, torch.ones_like(p))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("prec,flags", [("mixed", 0), ("mixed_mg", 0), ("fp64", 0x200)])
+def test_non_finite_source(value, prec, flags):
+    """One non-finite cell: reported, DP = 0 and p untouched."""
+    src = torch.randn(48, 40, 56, dtype=torch.float64, device="cuda")
+    src[3, 7, 11] = value
+    DP, p, info = _solve(src, (0.31, 0.17, 0.23), prec, flags=flags)
+    assert info.status == 5
+    assert float(DP.abs().max()) == 0.0 and torch.equal(p, torch.ones_like(p))
