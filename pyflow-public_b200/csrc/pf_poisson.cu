@@ -1886,6 +1886,26 @@ struct PlanLayout {
     SpectralPlan sp;  // on: the direct solve, with FP64 passes behind it
 };
 
+// The two slots at the end of a plan's workspace that are filled once: the
+// direct solve's tables, then the coarsest pseudo-inverse and the grid-barrier
+// words.  (The region R is rewritten every step.)
+static char* plan_tables(const pf_grid* g, int prec, void* ws) {
+    return (char*)ws + step_plan_ws_bytes(g, prec) - spectral_table_bytes(g) -
+           (prec == PF_MIXED_MG ? kPlanPinvBytes + kMgBarrierBytes : 0);
+}
+
+// PF_MIXED_MG: the multigrid of grids that coarsen, its vectors in region R.
+static int plan_mg(const pf_grid* g, int prec, void* ws, char* R, MgPlan* mg) {
+    const size_t n = (size_t)g->nx * g->ny * g->nz;
+    if (prec != PF_MIXED_MG || mg_region_bytes(g) > 9 * align256(n * sizeof(double))) return PF_OK;
+    const int e = mg_setup(g, R, mg);
+    if (e != PF_OK && e != PF_ERR_BAD_ARG) return e;
+    char* end = (char*)ws + step_plan_ws_bytes(g, prec);
+    if (mg->L && mg->pinv) mg->pinv = (float*)(end - kPlanPinvBytes - kMgBarrierBytes);
+    if (mg->L) mg->gbar = (unsigned*)(end - kMgBarrierBytes);
+    return PF_OK;
+}
+
 static int plan_layout(const pf_grid* g, int prec, double min_res, const double* DP, void* ws,
                        PlanLayout* L) {
     L->d = Dims{g->nx, g->ny, g->nz, (long long)g->nx * g->ny * g->nz};
@@ -1906,26 +1926,30 @@ static int plan_layout(const pf_grid* g, int prec, double min_res, const double*
     L->mg = MgPlan();
     L->sp = SpectralPlan();
     if (prec != PF_FP64 && !mg_cycles_serve(g, prec)) {
-        char* tables = (char*)ws + step_plan_ws_bytes(g, prec) - spectral_table_bytes(g) -
-                       (prec == PF_MIXED_MG ? kPlanPinvBytes + kMgBarrierBytes : 0);
+        char* tables = plan_tables(g, prec, ws);
         if (spectral_applies(g, min_res, DP, tables))
             return spectral_setup(g, tables, &L->sp) == cudaSuccess ? PF_OK : PF_ERR_CUDA;
     }
-    // PF_MIXED_MG: multigrid-preconditioned inner passes when the grid
-    // coarsens (vectors in the region of the FP32 solver vectors)
-    if (prec == PF_MIXED_MG && mg_region_bytes(g) <= 9 * align256(n * sizeof(double))) {
-        const int e = mg_setup(g, L->R, &L->mg);
-        if (e != PF_OK && e != PF_ERR_BAD_ARG) return e;
-        // the pseudo-inverse lives in the last slot of the workspace, outside
-        // the region the predictor overwrites, and is computed once here
-        if (L->mg.L && L->mg.pinv)
-            L->mg.pinv = (float*)((char*)ws + step_plan_ws_bytes(g, prec) - kPlanPinvBytes -
-                                  kMgBarrierBytes);
-        // the grid-barrier words too: the region is rewritten every step
-        if (L->mg.L)
-            L->mg.gbar = (unsigned*)((char*)ws + step_plan_ws_bytes(g, prec) - kMgBarrierBytes);
-    }
-    return PF_OK;
+    return plan_mg(g, prec, ws, L->R, &L->mg);
+}
+
+// Fills what the solvers keep in the workspace of a plan: for every solver that
+// serves the grid, not only the one P chose, since a later plan of the same
+// member (fresh == 0, nothing filled then) may choose another, by its tolerance
+// or PF_MG_COOP.
+static int plan_fill(const pf_grid* g, int prec, const double* DP, void* ws, const PlanLayout& P,
+                     cudaStream_t s) {
+    if (prec == PF_FP64) return PF_OK;
+    SpectralPlan sp;
+    MgPlan mg;
+    char* tables = plan_tables(g, prec, ws);
+    if (spectral_applies(g, kSpectralMinTol, DP, tables) &&
+        (spectral_setup(g, tables, &sp) != cudaSuccess ||
+         spectral_enqueue_tables(sp, s) != cudaSuccess))
+        return PF_ERR_CUDA;
+    const int rc = plan_mg(g, prec, ws, P.R, &mg);
+    if (rc != PF_OK) return rc;
+    return mg.L ? mg_enqueue_setup(mg, s) : PF_OK;
 }
 
 // The monitor statistics with the solve's result next to them, after node
@@ -2280,9 +2304,7 @@ int step_plan_create(const pf_grid* g, int prec, int rk4, double* u, double* v,
     if (c && c->kind == PF_CLOSURE_MLP && mlp_prepare() != cudaSuccess) return PF_ERR_CUDA;
     cudaStream_t cs;
     if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) return PF_ERR_CUDA;
-    if ((P.mg.L && mg_enqueue_setup(P.mg, cs) != PF_OK) ||
-        (P.sp.on && spectral_enqueue_tables(P.sp, cs) != cudaSuccess) ||
-        cudaStreamSynchronize(cs) != cudaSuccess) {
+    if (plan_fill(g, prec, DP, ws, P, cs) != PF_OK || cudaStreamSynchronize(cs) != cudaSuccess) {
         cudaStreamDestroy(cs);
         return PF_ERR_CUDA;
     }
@@ -2330,7 +2352,7 @@ int batch_plan_create(int prec, int rk4, const pf_batch_member* m, int count, vo
     if (count < 1 || count > kMaxBatch) return PF_ERR_BAD_ARG;
     PlanLayout* P = new PlanLayout[count];
     int rc = PF_OK;
-    for (int r = 0; r < count && rc == PF_OK; ++r) 
+    for (int r = 0; r < count && rc == PF_OK; ++r)
         rc = plan_layout(&m[r].grid, prec, m[r].min_res, m[r].DP, m[r].ws, &P[r]);
     if (rc != PF_OK) { delete[] P; return rc; }
     // the requests' solves run as parallel branches: their mid levels stay on
@@ -2353,9 +2375,7 @@ int batch_plan_create(int prec, int rk4, const pf_batch_member* m, int count, vo
     // member carried over from an earlier plan may still be computing there
     // and is not touched
     for (int r = 0; r < count && rc == PF_OK; ++r)
-        if (m[r].fresh && ((P[r].mg.L && mg_enqueue_setup(P[r].mg, cs) != PF_OK) ||
-                           (P[r].sp.on && spectral_enqueue_tables(P[r].sp, cs) != cudaSuccess)))
-            rc = PF_ERR_CUDA;
+        if (m[r].fresh) rc = plan_fill(&m[r].grid, prec, m[r].DP, m[r].ws, P[r], cs);
     if (rc == PF_OK && cudaStreamSynchronize(cs) != cudaSuccess) rc = PF_ERR_CUDA;
     StepPlan* plan = new StepPlan();
     prof_suspend(true);

@@ -160,3 +160,52 @@ def test_request_sharding_two_ranks_gloo():
         a, b = allv
         assert not set(a) & set(b) and sorted(a + b) == list(range(40))
         assert work == total
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(64, 64, 64), (24, 20, 36)])
+@pytest.mark.parametrize("change", ["to cycles", "to direct", "looser", "tighter"])
+def test_carried_member_whose_solver_changes(monkeypatch, shape, change):
+    """A member carried over into a plan that solves its pressure equation
+    another way (PF_MG_COOP set or unset in between, another tolerance) steps
+    bitwise like a StepPlan of its own: what either solver keeps in the
+    workspace is filled when the member first joins a plan.  (The workspaces
+    start as NaN.)"""
+    import pyflow_b200.initial as ic
+    from pyflow_b200.plan import BatchPlan, Member, StepPlan
+    sp = tuple(2 * np.pi / n for n in shape)
+    f0 = [torch.tensor(a, device="cuda") for a in ic.spectral_velocity(shape, k0=4.0, seed=3)]
+    f = [t.clone() for t in f0] + [torch.zeros_like(f0[0]), torch.zeros_like(f0[0])]
+    env = {"to cycles": (None, "0"), "to direct": ("0", None)}.get(change, (None, None))
+    tol = {"looser": (5e-13, 1e-10), "tighter": (1e-10, 5e-13)}.get(change, (1e-10, 1e-10))
+
+    def use(q):
+        monkeypatch.delenv("PF_MG_COOP", raising=False)
+        if env[q] is not None:
+            monkeypatch.setenv("PF_MG_COOP", env[q])
+
+    use(0)
+    m = Member(*f, sp, 0.01, 1.0, 0.004, min_res=tol[0], max_it=3000, prec="mixed_mg")
+    m.ws.fill_(255)
+    torch.cuda.synchronize()
+    first = BatchPlan([m])
+    first.launch(1)
+    torch.cuda.synchronize()
+    first.close()
+    use(1)
+    m.consts = m.consts[:3] + (tol[1],) + m.consts[4:]
+    g = [t.clone() for t in f]
+    own = StepPlan(*g, sp, 0.01, 1.0, 0.004, min_res=tol[1], max_it=3000, prec="mixed_mg")
+    second = BatchPlan([m])
+    assert not m.fresh
+    for _ in range(2):
+        second.launch(1)
+        own.launch(1)
+        torch.cuda.synchronize()
+        a, b = m.stats(), own.stats()
+        assert a["status"] == 0 and a["max_res"] <= tol[1]
+        assert a["iterations"] == b["iterations"]
+        for x, y in zip(f, g):
+            assert torch.equal(x, y)
+    second.close()
+    own.close()
