@@ -231,7 +231,8 @@ class SlabDomain:
     def solve(self):
         """solver_bicgstab.solve over the slabs: DP from the divergence held
         in ``div``; returns a SolveInfo (max_res, iterations, status)."""
-        if isinstance(self.T, LocalSlabs):
+        # (a transport derived from LocalSlabs carries its own exchanges)
+        if type(self.T) is LocalSlabs:
             info = self._solve_local()
             if info is not None:
                 return info

@@ -159,3 +159,36 @@ def test_slab_local_solve_is_the_phases(R, shape, max_it):
         out.append((D.gather("DP"), D.gather("u"), info.iterations, info.max_res, info.status))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert out[0][2:] == out[1][2:]
+
+
+def test_slab_transport_of_a_subclass_is_used():
+    """A transport derived from LocalSlabs carries the solve's exchanges and
+    gathers (one pp and one s exchange per iteration, three gathers and the
+    first), with the results of LocalSlabs itself."""
+    from pyflow_b200.slab import LocalSlabs, SlabDomain
+
+    class Counting(LocalSlabs):
+        calls, gathers = 0, 0
+
+        def exchange(self, *a, **k):
+            self.calls += 1
+            return super().exchange(*a, **k)
+
+        def allgather(self, *a, **k):
+            self.gathers += 1
+            return super().allgather(*a, **k)
+
+    shape = (24, 16, 20)
+    sp = tuple(2 * np.pi / n for n in shape)
+    f0 = _fields(shape, seed=4)
+    out = []
+    for T in (Counting(2), LocalSlabs(2)):
+        D = SlabDomain(shape, sp, 0.01, 1.0, 0.005, T, min_res=1e-10, max_it=5000, poll=1)
+        D.set_state(*f0)
+        info = D.forward_step()
+        assert info.status == 0
+        out.append((D.gather("DP"), D.gather("u"), info.iterations))
+        if isinstance(T, Counting):
+            assert T.calls >= 2 * info.iterations and T.gathers >= 3 * info.iterations + 1
+    assert out[0][2] == out[1][2]
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
