@@ -26,7 +26,7 @@
  *    fast transforms, check the true residual, and iterate (in FP64) only if
  *    it misses the tolerance; the solve then counts as one iteration.  (Of
  *    the grids that coarsen, PF_MIXED_MG solves those of more than 2^15 cells
- *    directly, and none when PF_MG_COOP is set in the environment.)
+ *    directly, and none when PF_MG_COOP has a value in the environment, 0 included.)
  */
 #ifndef PYFLOW_B200_H
 #define PYFLOW_B200_H

@@ -1659,7 +1659,10 @@ static cudaError_t mg_attrs() {
     return cudaSuccess;
 }
 
-bool mg_cycles_requested() { return std::getenv("PF_MG_COOP") != nullptr; }
+bool mg_cycles_requested() {
+    const char* env = std::getenv("PF_MG_COOP");
+    return env && *env;
+}
 
 int mg_setup(const pf_grid* g, void* region, MgPlan* P) {
     P->L = mg_levels(g, P->lv, &P->B);

@@ -64,9 +64,10 @@ constexpr size_t kMgBarrierBytes = 256;
 int mg_levels(const pf_grid* g, MgLevel* lv, int* bottom);
 // FP32 bytes of the Krylov vectors and the coarse levels (0 if L == 0).
 size_t mg_region_bytes(const pf_grid* g);
-// True when PF_MG_COOP is set in the environment (0 or 1: how the V-cycle's
+// True when PF_MG_COOP has a value in the environment (0 or 1: how the V-cycle's
 // mid levels run): PF_MIXED_MG then iterates with V-cycles on every grid that
-// coarsens, also where the direct solve (pf_spectral.cuh) would serve.
+// coarsens, also where the direct solve (pf_spectral.cuh) would serve, so that 0
+// and 1 give the same bits.  An empty value is as none.
 bool mg_cycles_requested();
 // Carve the vectors from `region` (mg_region_bytes long, 256-byte aligned).
 int mg_setup(const pf_grid* g, void* region, MgPlan* P);

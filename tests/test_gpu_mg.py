@@ -190,3 +190,13 @@ def test_captured_vcycles_leave_for_fp64_passes(n, min_res, max_it):
         for x, y in zip(a[:3], b[:3]):
             assert (x - y).abs().max().item() <= 1e-11 * y.abs().max().item()
     plan.close()
+
+
+def test_mg_empty_coop_variable_is_unset(monkeypatch):
+    """PF_MG_COOP without a value is the same as no PF_MG_COOP: the direct
+    solve (one iteration) where it serves."""
+    monkeypatch.setenv("PF_MG_COOP", "")
+    src, sp = _source((64, 64, 64), seed=2)
+    DP, info = _solve(src, sp, "mixed_mg")
+    assert info.status == 0 and info.iterations == 1
+    assert _true_residual(src, DP, sp) <= 1e-10
