@@ -207,3 +207,61 @@ def test_plan_sfs_matches_forward_step(prec, closure):
         ops.forward_step(*c, sp, nu, 1.0, dt, min_res=1e-10, max_it=5000, prec=prec,
                          warm=prec != "fp64")
     assert (c[0] - b[0]).abs().max().item() > 1e-9
+
+
+@pytest.mark.parametrize("shape", [(24, 20, 36), (21, 20, 33)])
+def test_captured_fp32_passes_match_host_solve(shape):
+    """FP32 passes alone (small grids reach the tolerance with them) over
+    several launches of one graph, each from the previous step's DP."""
+    import pyflow_b200.initial as ic
+    import pyflow_b200.ops as ops
+    from pyflow_b200.plan import StepPlan
+    sp, tol = tuple(2 * np.pi / n for n in shape), 5e-13
+    f0 = [torch.tensor(x, device="cuda") for x in ic.spectral_velocity(shape, k0=4.0, seed=5)]
+    a = [t.clone() for t in f0] + [torch.zeros_like(f0[0]), torch.zeros_like(f0[0])]
+    b = [t.clone() for t in a]
+    plan = StepPlan(*b, sp, 0.01, 1.0, 0.005, min_res=tol, max_it=5000, prec="mixed")
+    for _ in range(3):
+        info = ops.forward_step(*a, sp, 0.01, 1.0, 0.005, min_res=tol, max_it=5000, prec="mixed",
+                                warm=True)
+        plan.launch(1)
+        torch.cuda.synchronize()
+        st = plan.stats()
+        assert info.status == 0 and st["status"] == 0 and st["max_res"] <= tol
+        assert int(st["iterations"]) == info.iterations > 1
+        for x, y in zip(a[:3], b[:3]):
+            assert (x - y).abs().max().item() <= 1e-12 * y.abs().max().item()
+    plan.close()
+
+
+def test_captured_refinement_without_multigrid_switches_to_fp64():
+    """A tolerance at FP64 rounding, without multigrid: FP32 passes until two
+    in a row gain less than 2x, then FP64 passes (the IF node's other branch),
+    in the graph as in the host-driven solve, whose kernel counts show both
+    kinds: same passes, iterations, residual and velocity.  The second launch
+    begins with FP32 passes again."""
+    import pyflow_b200.initial as ic
+    import pyflow_b200.ops as ops
+    import pyflow_b200.profiling as prof
+    from pyflow_b200.plan import StepPlan
+    shape, tol, max_it = (64, 64, 64), 1e-15, 3000
+    sp = tuple(2 * np.pi / n for n in shape)
+    f0 = [torch.tensor(x, device="cuda") for x in ic.spectral_velocity(shape, k0=4.0, seed=6)]
+    a = [t.clone() for t in f0] + [torch.zeros_like(f0[0]), torch.zeros_like(f0[0])]
+    b = [t.clone() for t in a]
+    plan = StepPlan(*b, sp, 0.01, 1.0, 0.005, min_res=tol, max_it=max_it, prec="mixed")
+    for _ in range(2):
+        prof.enable(True)
+        info = ops.forward_step(*a, sp, 0.01, 1.0, 0.005, min_res=tol, max_it=max_it,
+                                prec="mixed", warm=True)
+        kt = prof.read()
+        prof.enable(False)
+        assert kt["bicg_init_f32"]["launches"] > 1 and kt["bicg_init_f64"]["launches"] > 1
+        plan.launch(1)
+        torch.cuda.synchronize()
+        st = plan.stats()
+        assert int(st["status"]) == info.status and st["max_res"] == info.max_res
+        assert int(st["iterations"]) == info.iterations
+        for x, y in zip(a[:3], b[:3]):
+            assert (x - y).abs().max().item() <= 1e-12 * y.abs().max().item()
+    plan.close()

@@ -218,3 +218,67 @@ def test_non_finite_source(value, prec, flags):
     DP, p, info = _solve(src, (0.31, 0.17, 0.23), prec, flags=flags)
     assert info.status == 5
     assert float(DP.abs().max()) == 0.0 and torch.equal(p, torch.ones_like(p))
+
+
+def test_tight_tolerance_is_reached():
+    """Below the direct solve's tolerance the iterations reach theirs: the true
+    residual (evaluated again: a few roundings of the operator's largest
+    terms, kappa times |b|), and with it the solution: |error| <= |r| / least
+    eigenvalue in the 2-norm, |r| <= sqrt(N) max|r|."""
+    import pyflow_b200.ops as ops
+    n, h, tol, c1 = 24, 0.1, 2e-13, 1.3 / 0.01
+    a = np.random.default_rng(3).standard_normal((n,) * 3)
+    a -= a.mean()
+    src, sp = torch.tensor(a, device="cuda"), (h,) * 3
+    DP, _, info = _solve(src, sp, "mixed", tol=tol)
+    assert info.status == 0 and info.iterations > 1
+    s2 = np.sin(np.pi / n) ** 2
+    b = src * c1 * -(h ** 3)
+    res = float((b - ops.laplace_apply(DP, sp)).abs().max() / b.abs().max())
+    assert res <= tol + 8 * 2.0 ** -53 * 3 / s2
+    got, want = DP.cpu().numpy(), _exact(a, sp)
+    got -= got.mean()
+    bound = tol * np.sqrt(a.size) * np.abs(a).max() * c1 * h ** 2 / (4 * s2)
+    assert np.linalg.norm(got - want) <= bound + 1e-15 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("shape", [(40, 36, 24), (21, 20, 33)])
+def test_correction_taken_back_costs_its_roundings(shape):
+    """The flattened box of test_plan_takes_the_correction_back, first step:
+    the graph's velocity went through the rejected correction c0 = dt/rho grad
+    DP0 and back, the host-driven one did not, and both then take the same
+    correction.  Each of the two extra operations rounds a value of at most
+    |u| + 2 |c0| once, and differing inputs of the last one can round apart
+    once more: 4 units of 2^-53 of |u| + 2 |c0| + |c1| (c1: the final
+    correction), beside what the two DP themselves differ by; the pressure
+    likewise with DP0 and DP1."""
+    import pyflow_b200.ops as ops
+    from pyflow_b200.plan import StepPlan
+    sp, dt = (0.2, 0.25, 2e-6), 1e-7
+    rng = np.random.default_rng(5)
+    k = [2 * np.pi * np.arange(n) / n for n in shape[:2]]
+    f0 = [np.broadcast_to((np.sin(k[0] + a)[:, None] * np.cos(k[1] + b)[None, :])[..., None], shape)
+          for a, b in rng.uniform(0, 6, (3, 2))]
+    f0 = [torch.tensor(np.ascontiguousarray(x), device="cuda") for x in f0]
+    z = lambda: torch.zeros_like(f0[0])  # noqa: E731
+    a, b = [t.clone() for t in f0] + [z(), z()], [t.clone() for t in f0] + [z(), z()]
+    info = ops.forward_step(*a, sp, 0.0, 1.0, dt, min_res=1e-10, max_it=12, prec="mixed")
+    plan = StepPlan(*b, sp, 0.0, 1.0, dt, min_res=1e-10, max_it=12, prec="mixed")
+    plan.launch(1)
+    torch.cuda.synchronize()
+    assert plan.stats()["status"] != 0 and info.status != 0
+    plan.close()
+    # the rejected correction: the direct solve of the same divergence alone
+    c = [t.clone() for t in f0]
+    ops.predictor_step(*c, sp, 0.0, 1.0, dt, prec="mixed")
+    DP0, p = z(), z()
+    ops.bicgstab_solve(ops.div_vel(*c, sp), DP0, p, sp, 1.0, dt, 1e-10, 1, prec="mixed")
+
+    def grad(f, d):
+        return dt * (f - f.roll(1, d)) / sp[d]
+    for d in range(3):
+        bound = 4 * 2.0 ** -53 * (c[d].abs() + 2 * grad(DP0, d).abs() + grad(a[4], d).abs())
+        bound += grad(a[4] - b[4], d).abs()
+        assert bool(((a[d] - b[d]).abs() <= bound).all())
+    bound = 4 * 2.0 ** -53 * (2 * DP0.abs() + a[4].abs()) + (a[4] - b[4]).abs()
+    assert bool(((a[3] - b[3]).abs() <= bound).all())
