@@ -21,12 +21,14 @@
  *    BiCGStab is unpreconditioned); it needs the grid to halve in every
  *    dimension (while all are even) down to at most 4096 cells, and otherwise
  *    runs the PF_MIXED passes.  Both mixed forms converge to the same FP64
- *    tolerance.  Where every extent is at most 2048 and the tolerance at
- *    least 1e-12, both first solve the pressure equation directly by FP64
+ *    tolerance.  Where every extent is at most 2048 (with a factor 5 1280,
+ *    else with a factor 3 1536, else with a factor 7 1792) and the tolerance
+ *    at least 1e-12, both first solve the pressure equation directly by FP64
  *    fast transforms, check the true residual, and iterate (in FP64) only if
  *    it misses the tolerance; the solve then counts as one iteration.  (Of
  *    the grids that coarsen, PF_MIXED_MG solves those of more than 2^15 cells
- *    directly, and none when PF_MG_COOP has a value in the environment, 0 included.)
+ *    directly, and none when PF_MG_COOP has a value in the environment, 0
+ *    included.  DP in the source's own buffer is solved by iterations.)
  */
 #ifndef PYFLOW_B200_H
 #define PYFLOW_B200_H

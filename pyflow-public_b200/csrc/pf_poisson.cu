@@ -904,7 +904,8 @@ constexpr int kPassBlocks = 592;
 //            scale grad DP (src/data/domain.py:394-402).
 // With both, the correction does not wait for the check: where it then fails
 // (a source with a mean, a tolerance below the transforms' rounding),
-// project_undo takes it back before FP64 BiCGStab passes go on from DP.  80
+// project_undo takes it back before FP64 BiCGStab passes go on from DP (u and p
+// keep at most two roundings of |u| + 2 |scale grad DP| from that).  80
 // bytes per cell, 26.6 us at 128^3 and 7.5 at 64^3 (6.3 TB/s of L2 and HBM at
 // 128^3); as three kernels (96 bytes) with an IF node between the check and the
 // correction it took 57 and 26 us of a step.
@@ -1180,21 +1181,22 @@ static int run_iterations(const Dims& d, const LapCoef<T>& cf,
 }
 
 // PF_MIXED_MG grids that keep the V-cycle iterations where the direct solve
-// would serve too: all that coarsen when PF_MG_COOP asks for them, and those
-// of at most 2^15 cells.  At 32^3 a captured step takes 0.57 ms with the
-// V-cycles and 0.10 ms with the direct solve, but any change of DP, however
-// small, flips roundings of the FP32 stages, and on these coarse grids (few
-// points per wave, large steps) the two solvers' trajectories part within a
-// request: after 10 steps the velocities differ by 3e-9 (2-norm; by 8e-15
-// after the first), against at most 9e-11 after 5 steps at 128^3, 1.9e-10
-// after 3 at 90x77x63 and 2e-10 in ensembles up to 192^3 after 4 (single cells
-// beside a flip at a large velocity by up to 8e-8).  Requests this small keep
-// the results they have.
-constexpr long long kDirectMinCells = 1LL << 15;
+// would serve too: all that coarsen when PF_MG_COOP asks for them, and those of
+// at most 2^15 cells.  The bound keeps the results that such requests had before
+// there was a direct solve; it is not the faster choice (a captured 32^3 step
+// takes 0.55 ms with the V-cycles, 0.10 ms direct) nor the more accurate one.
+// Any change of DP, however small, flips roundings of the FP32 stages, and the
+// flips grow: at 32^3, the one size measured below the bound, the velocities of
+// the two solvers differ by up to 3e-9 after 10 steps (2-norm; 8e-15 after the
+// first), where either is 1.6e-8 from the FP64 form.  Measured above it: 9e-11 after 5
+// steps at 128^3, 1.9e-10 after 3 at 90x77x63, 2e-10 after 4 in ensembles up to
+// 192^3 (single cells beside a flip at a large velocity by up to 8e-8).
+// PF_MIXED, and grids of any size that do not coarsen, solve directly.
+constexpr long long kCyclesMaxCells = 1LL << 15;
 
 static bool mg_cycles_serve(const pf_grid* g, int prec) {
     if (prec != PF_MIXED_MG || mg_region_bytes(g) == 0) return false;
-    return mg_cycles_requested() || (long long)g->nx * g->ny * g->nz <= kDirectMinCells;
+    return mg_cycles_requested() || (long long)g->nx * g->ny * g->nz <= kCyclesMaxCells;
 }
 
 int bicgstab_solve(const pf_grid* g, int prec, double rho, double dt,

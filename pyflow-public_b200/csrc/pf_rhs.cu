@@ -878,7 +878,9 @@ static cudaError_t grouped_prepare() {
 }
 
 // Job of one request for one stage (the arguments the single-request
-// predictor_impl passes to that stage).
+// predictor_impl passes to that stage; the x split is make_tiling's, made to fill
+// the GPU by one request: rhs_tiling, for lone launches, was not tried for the
+// tiles of several.  Any split gives the same bits).
 template <typename T, typename TI>
 static StageJob<T, TI> make_job(const GroupMember& m, const TI* in_u, const TI* in_v,
                                 const TI* in_w, T* st, T* acc, long long tile0) {

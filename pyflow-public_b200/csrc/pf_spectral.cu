@@ -22,8 +22,8 @@
 // element-wise accesses conflict.  A thread holds 8 complex values.  In the x
 // and y passes a line pair is two neighbouring cells in z, and a block's L = 8
 // pairs read and write runs of 128 bytes; in the z pass the rows themselves
-// are contiguous.  Extents 2^k, 3 2^k and 5 2^k from 32 to 1024 have kernels of
-// their own (pf_spectral_fast.cu).
+// are contiguous.  The multiples of 32 among 2^k, 3 2^k and 5 2^k up to 1024 have
+// kernels of their own (pf_spectral_fast.cu); 48 and 80, for example, do not.
 #include <algorithm>
 #include <cmath>
 

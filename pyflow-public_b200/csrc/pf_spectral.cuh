@@ -6,7 +6,12 @@
 
 namespace pf {
 
-constexpr int kSpectralMaxN = 2048;   // longest extent: its tile fits one block's shared memory
+// Longest extent.  A stage's butterflies run in one go, at most 8 values a
+// thread, so radix 3, 5 and 7 stages (6, 5 and 7 values) need more threads a line
+// than n / 8, and a block (512 threads, at least two line pairs) takes extents
+// with a factor 5 up to 1280, else with a factor 3 up to 1536, else with a factor
+// 7 up to 1792, all others to 2048 (spectral_applies).
+constexpr int kSpectralMaxN = 2048;
 constexpr int kSpectralMaxStages = 12;
 
 // The tightest relative residual the direct solve is asked for: its own

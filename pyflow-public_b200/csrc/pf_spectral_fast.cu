@@ -1,6 +1,6 @@
 // pf_spectral_fast.cu -- the transform passes of pf_spectral.cu for extents
-// 2^k, 3 2^k and 5 2^k (multiples of 32 up to 1024) with every index known at
-// compile time.
+// 2^k, 3 2^k and 5 2^k that are multiples of 32, up to 1024, with every index
+// known at compile time.
 //
 // The pass of any extent (pf_spectral.cu) is bound by the shared-memory pipe
 // (77-81 % busy at 256^3) and by integer instructions: a value goes through
