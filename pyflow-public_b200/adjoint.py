@@ -176,13 +176,13 @@ def predictor_vjp(state, lam, spacing, mu, rho, dt, sfs=None, rk4=True):
     for t in (*state, *lam):
         ops._check(t, state[0].shape, torch.float64, "state and adjoint")
     u = state[0]
-    if sfs is not None:
+    if sfs is not None and rk4:  # (Euler's only stage state is the input: not read)
         ops._check(sfs, (6,) + tuple(u.shape), torch.float64, "sfs")
     g = ops.grid(u.shape, spacing)
     need = _lib.pf_predictor_vjp_workspace_bytes(ctypes.byref(g))
     ws = torch.empty(need, dtype=torch.uint8, device=u.device)
     out = tuple(torch.empty_like(u) for _ in range(3))
-    lamF = torch.empty_like(sfs) if sfs is not None else None
+    lamF = u.new_empty((6,) + tuple(u.shape)) if sfs is not None else None
     L.check("pf_predictor_vjp", _lib.pf_predictor_vjp(
         ctypes.byref(g), 1 if rk4 else 0, *(ops._p(t) for t in (*state, *lam)), float(mu),
         float(rho), float(dt), ops._p(sfs), *(ops._p(t) for t in out), ops._p(lamF), ops._p(ws),

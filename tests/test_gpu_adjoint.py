@@ -174,3 +174,20 @@ def test_predictor_vjp_of_an_adjoint_that_is_the_state(A, rk4, which):
         assert torch.equal(x, y)
     for x, y in zip(state, keep):
         assert torch.equal(x, y)
+
+
+def test_euler_vjp_takes_stresses_of_any_layout(A):
+    """The Euler form's gradient does not read the stresses: a strided or FP32
+    stress tensor gives the FP64 contiguous one's result, in a contiguous
+    FP64 tensor."""
+    rng = np.random.default_rng(4)
+    shape, sp = (7, 9, 12), (0.31, 0.17, 0.23)
+    r = lambda *s: torch.tensor(rng.standard_normal(s), device="cuda")  # noqa: E731
+    state, lam = [r(*shape) for _ in range(3)], [r(*shape) for _ in range(3)]
+    sfs = r(6, *shape)
+    want, F = A.step_vjp(state, lam, sp, 0.013, 1.2, 0.01, sfs=sfs, rk4=False)
+    for other in (sfs.permute(0, 3, 2, 1).contiguous().permute(0, 3, 2, 1), sfs.float()):
+        out, G = A.step_vjp(state, lam, sp, 0.013, 1.2, 0.01, sfs=other, rk4=False)
+        assert G.dtype == torch.float64 and G.is_contiguous() and torch.equal(F, G)
+        for x, y in zip(out, want):
+            assert torch.equal(x, y)
